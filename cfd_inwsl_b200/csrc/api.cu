@@ -1484,8 +1484,8 @@ extern "C" int cfd_accuracy_test(int inter_method, int n, double h, const double
 
 namespace cfd {
 // Default cells per CTA segment along direction d for the tile shapes that
-// launch_sweep picks for this configuration: about six waves of CTAs over the
-// 148 SMs. Shared with the allocation-free entry point (noalloc.cu).
+// launch_sweep picks for this configuration. Shared with the allocation-free
+// entry point (noalloc.cu).
 int default_seg_len_for(const cfd_config *cfg, int fam, bool strict, int d)
 {
     int n = cfg->n[d];
@@ -1513,6 +1513,31 @@ int default_seg_len_for(const cfd_config *cfg, int fam, bool strict, int d)
     const long long target = mixed_x ? 148LL * 2 * 3 : 148LL * 2 * 6;
     int seg = n;
     while (blocks_per_seg * ((n + seg - 1) / seg) < target && seg > 4 * S) seg = (seg + 1) / 2;
+    if (blocks_per_seg * ((n + seg - 1) / seg) >= target) return seg;
+    // Grids too small for that: whole chunks per segment, by cost. A CTA's is
+    // its chunks, the first one's second pass over the extra faces (nearly a
+    // chunk's latency) and half a chunk of set-up, times its waves over 3
+    // resident CTAs per SM; below one wave a chunk takes about 4 us with one
+    // CTA per SM and hardly longer with three, so the longest CTA counts and
+    // one-chunk segments win; above it the mean counts, and a wave that is
+    // nearly empty costs about half a full one. Fitted on sweeps timed over 1
+    // to 64 chunks a segment from a 400-cell line to 512^2. Stopping at four
+    // chunks left a 64^2 grid 8 CTAs and a 400-cell line one: 24 strict steps
+    // of 64^2 4.10 -> 1.93 ms, 300 of 400 cells 31.3 -> 14.1 ms.
+    double best = 1e300;
+    for (int s = S; ; s += S) {
+        const int len = s < n ? s : n;
+        const long long nseg = (n + len - 1) / len;
+        const int tail = n - (int)(nseg - 1) * len;
+        const double k = (len + S - 1) / S, w = (double)(blocks_per_seg * nseg) / (148.0 * 3);
+        const double mean = ((double)(nseg - 1) * k + (tail + S - 1) / S) / (double)nseg;
+        const double cost = w <= 1.0 ? (k + 1.3) * (0.85 + 0.3 * w) : (mean + 0.85) * (0.5 * (std::ceil(w) + w) + 0.3);
+        if (cost < best) {
+            best = cost;
+            seg = len;
+        }
+        if (len == n) break;
+    }
     return seg;
 }
 
