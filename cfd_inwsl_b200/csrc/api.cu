@@ -219,6 +219,37 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
             for (int j = 0; j < 3; j++)
                 if (__double_as_longlong(Q[j]) != __double_as_longlong(A[j] / bs)) cnt++;
         }
+        // the sweeps' branch-free operations where they accept the operands:
+        // the pair above, and operands next to the ends of a binade (all-ones
+        // significands, one ulp above a power of two) where a reciprocal or a
+        // root lies nearest a rounding boundary
+        {
+            const unsigned long long k = splitmix64(st) % 8;
+            const int e = (int)(splitmix64(st) % 121) - 60;
+            const unsigned long long m = (1ULL << 52) - 1, low = splitmix64(st) % 16;
+            const unsigned long long mant = (k == 0) ? m - low : (k == 1) ? low : (splitmix64(st) & m);
+            const double bs = __longlong_as_double((long long)(((unsigned long long)(1023 + e) << 52) | mant));
+            const double bp = (k < 4) ? bs : b;
+            {
+                cfd::OpsSpec o;
+                const double r = o.rcp(bp);
+                if (o.ok && __double_as_longlong(r) != __double_as_longlong(1.0 / bp)) cnt++;
+                const double q = o.div_y(a, bp, r);
+                if (o.ok && __double_as_longlong(q) != __double_as_longlong(a / bp)) cnt++;
+            }
+            {
+                cfd::OpsSpec o;
+                const double q = o.div(a, bp);
+                if (o.ok && __double_as_longlong(q) != __double_as_longlong(a / bp)) cnt++;
+            }
+            {  // roots: as above, and next to the square of a rounding boundary
+                const double s = fabs(bp), hu = ldexp(1.0, ilogb(s) - 53);
+                const double x = (k & 1) ? fma(s, s, s * (2.0 * hu)) : s;
+                cfd::OpsSpec o;
+                const double r = o.sqrt(x);
+                if (o.ok && __double_as_longlong(r) != __double_as_longlong(sqrt(x))) cnt++;
+            }
+        }
     }
     if (cnt) atomicAdd(bad, cnt);
 }

@@ -149,6 +149,146 @@ CFD_HD void divs_rn(const double *a, const double *b, const double *y, double *q
 }
 
 // ---------------------------------------------------------------------------
+// Arithmetic policies of the pointwise functions below.
+//
+// OpsIeee divides and takes roots with the compiler's own operations, whose
+// special cases are branches. OpsSpec is for the sweeps: no branches, so that
+// the chains of a face (8 to 10 interpolations, two face states, a Riemann
+// flux) interleave in one straight piece of code. Each operation checks with
+// integer operations that its operands lie in the range its proof covers and
+// clears `ok` otherwise; the caller then discards the result and evaluates the
+// whole cell or face again with OpsIeee, out of line.
+//
+// Strict flavour: every result is the IEEE one. With y = RN(1/b) and q0 =
+// RN(a y), |a/b - q0| < 3/2 ulp, so if a/b lies within half an ulp of a
+// rounding boundary q0 is one of its two neighbours, and RN(q0 + (a - b q0) y),
+// the residual exact in an FMA, is RN(a/b) (P. Markstein, IBM J. Res. Develop.
+// 34(1), 1990). y comes from the hardware's reciprocal approximation by one
+// cubic (Halley) step, 1/b (1 - e^3) for a seed off by e; a further Markstein
+// step makes it RN(1/b) where 1/b itself is wanted. The root is Markstein's
+// s + (x - s^2) / (2 sqrt x) on a seed after one cubic step. Division: 6
+// operations on the FP64 pipe instead of about 14 issue slots and a branch;
+// cfd_check_division compares all of them with IEEE on the device.
+// Fast flavour: the same steps without the last correction where its own
+// arithmetic multiplies by reciprocals.
+// ---------------------------------------------------------------------------
+struct OpsIeee {
+    static constexpr bool spec = false;
+#if defined(CFD_FAST)
+    CFD_HD double rcp(double b) { return 1.0 / b; }
+    CFD_HD double div_y(double a, double, double y) { return a * y; }
+#if defined(__CUDACC__)
+    __device__ __forceinline__ double rsqrt(double x) { return ::rsqrt(x); }
+#endif
+#else
+    CFD_HD double rcp(double b) { return rcp_rn(b); }
+    CFD_HD double div_y(double a, double b, double y) { return div_rn(a, b, y); }
+#endif
+    CFD_HD double div(double a, double b) { return a / b; }
+    CFD_HD double div_pos(double a, double b) { return a / b; }
+    CFD_HD double sqrt(double x) { return ::sqrt(x); }
+    CFD_HD void need(bool) {}
+};
+
+#if defined(__CUDACC__)
+struct OpsSpec {
+    static constexpr bool spec = true;
+    bool ok = true;
+
+    __device__ __forceinline__ void need(bool c) { ok = ok & c; }
+    // 2^-400 <= x < 2^200 (false for negative, zero, non-finite): divisors and radicands
+    static __device__ __forceinline__ bool in_range(double x)
+    {
+        return (unsigned)__double2hiint(x) - (623u << 20) < (600u << 20);
+    }
+    // x = +-0 or 2^-800 <= |x| < 2^500: dividends, whose quotients and
+    // residuals then stay normal numbers
+    static __device__ __forceinline__ bool in_range_or_0(double x)
+    {
+        const unsigned t = (unsigned)__double2hiint(x) & 0x7fffffffu, lo = (unsigned)__double2loint(x);
+        return (t - (223u << 20) < (1300u << 20)) | ((t | lo) == 0u);
+    }
+    // 1/b to just over half an ulp: seed (relative error e) and y (1 + e + e^2).
+    // e + e^2 is rounded up: for a significand of all ones 1/b lies 2^-107
+    // above a rounding boundary, the one case in which the Markstein step
+    // does not recover from the neighbour below.
+    static __device__ __forceinline__ double rcp_near(double b)
+    {
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+        double e = fma(-b, y, 1.0);
+        e = __fma_ru(e, e, e);
+        return fma(y, e, y);
+    }
+    // RN(a/b) from y = 1/b, b > 0. The residual carries the sign that keeps a
+    // quotient of a zero dividend at that zero.
+    static __device__ __forceinline__ double quot(double a, double b, double y)
+    {
+        const double q = a * y;
+        return fma(-fma(b, q, -a), y, q);
+    }
+    __device__ __forceinline__ double rcp(double b)
+    {
+        need(in_range(b));
+        const double y = rcp_near(b);
+#if defined(CFD_FAST)
+        return y;
+#else
+        return fma(fma(-b, y, 1.0), y, y);
+#endif
+    }
+    __device__ __forceinline__ double div_y(double a, double b, double y)
+    {
+#if defined(CFD_FAST)
+        return a * y;
+#else
+        need(in_range_or_0(a));
+        return quot(a, b, y);
+#endif
+    }
+    // a / b for b > 0 (any other b takes the out-of-line path)
+    __device__ __forceinline__ double div(double a, double b)
+    {
+        need(in_range(b) & in_range_or_0(a));
+        return quot(a, b, rcp_near(b));
+    }
+    // the same where 2^-800 <= a < 2^500 is known
+    __device__ __forceinline__ double div_pos(double a, double b)
+    {
+        need(in_range(b));
+        return quot(a, b, rcp_near(b));
+    }
+    // 1/sqrt(x) seed and one cubic step's factor: y (1 + p) = 1/sqrt(x) (1 - O(e^3))
+    static __device__ __forceinline__ double rsqrt_seed(double x)
+    {
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        return y;
+    }
+    __device__ __forceinline__ double sqrt(double x)
+    {
+        need(in_range(x));
+        const double y = rsqrt_seed(x);
+        double g = x * y, h = 0.5 * y;
+        const double r = fma(-g, h, 0.5);
+        const double p = fma(1.5 * r, r, r);
+        g = fma(g, p, g);
+        h = fma(h, p, h);
+        return fma(fma(-g, g, x), h, g);
+    }
+#if defined(CFD_FAST)
+    __device__ __forceinline__ double rsqrt(double x)
+    {
+        need(in_range(x));
+        const double y = rsqrt_seed(x);
+        const double e = fma(-x * y, y, 1.0);
+        return fma(y, fma(0.375, e, 0.5) * e, y);
+    }
+#endif
+};
+#endif
+
+// ---------------------------------------------------------------------------
 // Five-point interpolators (zone_FD/src/include/interScheme.hpp).
 // q0..q4 are the five upwind-ordered point values; the result is the value at
 // the face between q2 and q3.
@@ -299,12 +439,8 @@ enum ResearchVariant : int {
 // keep-all test it is the rare path, and keeping it out of the unrolled face
 // code shortens the hot loop's instruction footprint (5.6% faster TENO5 + Roe
 // steps on B200).
-#if defined(__CUDACC__)
-static __host__ __device__ __noinline__
-#else
-CFD_HD
-#endif
-unsigned teno_z_flag(double b0, double b1, double b2, double tau, double c)
+template <class O>
+CFD_HD unsigned teno_z_flag_ops(double b0, double b1, double b2, double tau, double c, O &o)
 {
     const double eps = 1e-40;
     double t;
@@ -324,10 +460,11 @@ unsigned teno_z_flag(double b0, double b1, double b2, double tau, double c)
     t = 1.0 + r1; t *= t; b1 = t * t * t;
     t = 1.0 + r2; t *= t; b2 = t * t * t;
 #else
-    t = 1.0 + tau / (b0 + eps); t *= t; b0 = t * t * t;
-    t = 1.0 + tau / (b1 + eps); t *= t; b1 = t * t * t;
-    t = 1.0 + tau / (b2 + eps); t *= t; b2 = t * t * t;
+    t = 1.0 + o.div(tau, b0 + eps); t *= t; b0 = t * t * t;
+    t = 1.0 + o.div(tau, b1 + eps); t *= t; b1 = t * t * t;
+    t = 1.0 + o.div(tau, b2 + eps); t *= t; b2 = t * t * t;
 #endif
+    (void)o;
     double sumbeta = 0.0;
     sumbeta += b0; sumbeta += b1; sumbeta += b2;
     const double CT = c * sumbeta;
@@ -336,6 +473,24 @@ unsigned teno_z_flag(double b0, double b1, double b2, double tau, double c)
     if (b1 < CT) flag += 2;
     if (b2 < CT) flag += 4;
     return flag;
+}
+
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__
+#else
+CFD_HD
+#endif
+unsigned teno_z_flag(double b0, double b1, double b2, double tau, double c)
+{
+#if defined(__CUDA_ARCH__) && !defined(CFD_FAST)
+    // without branches where the operands allow it: shocked flows take this
+    // path often, and three IEEE divisions one after the other were its length
+    OpsSpec s;
+    const unsigned f = teno_z_flag_ops(b0, b1, b2, tau, c, s);
+    if (s.ok) return f;
+#endif
+    OpsIeee o;
+    return teno_z_flag_ops(b0, b1, b2, tau, c, o);
 }
 
 // The cut-off flag of a research variant (bit k set = stencil k cut), in the
@@ -541,8 +696,8 @@ unsigned research_flag(int variant, double q0, double q1, double q2, double q3, 
     }
 }
 
-template <int FAM>
-CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, double c, double kap = 0.0)
+template <int FAM, class O>
+CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, double c, double kap, O &o)
 {
     if constexpr (FAM == FAM_WCNS5) {
         // weno5_JSchen: omega_k = gamma_k / (eps + beta_k)^2, eps = 1e-6.
@@ -557,17 +712,17 @@ CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, doub
         double s0 = eps + b0, s1 = eps + b1, s2 = eps + b2;
         s0 *= s0; s1 *= s1; s2 *= s2;
         double w0 = (1.0 / 16.0) * (s1 * s2), w1 = (5.0 / 8.0) * (s0 * s2), w2 = (5.0 / 16.0) * (s0 * s1);
-        return (w0 * u0 + w1 * u1 + w2 * u2) / (w0 + w1 + w2);
+        return o.div(w0 * u0 + w1 * u1 + w2 * u2, w0 + w1 + w2);
 #else
         double s;
         // (1/16) / s^2 = RN(1 / s^2) / 16 exactly (a power-of-two scaling)
-        s = eps + b0; b0 = rcp_rn(s * s) * (1.0 / 16.0);
-        s = eps + b1; b1 = (5.0 / 8.0) / (s * s);
-        s = eps + b2; b2 = (5.0 / 16.0) / (s * s);
-        double sumbeta = 0.0, result = 0.0;
-        sumbeta += b0; sumbeta += b1; sumbeta += b2;
+        s = eps + b0; b0 = o.rcp(s * s) * (1.0 / 16.0);
+        s = eps + b1; b1 = o.div_pos(5.0 / 8.0, s * s);
+        s = eps + b2; b2 = o.div_pos(5.0 / 16.0, s * s);
+        double sumbeta = b0, result = 0.0;  // 0 + b0 = b0 (b0 > 0)
+        sumbeta += b1; sumbeta += b2;
         result += b0 * u0; result += b1 * u1; result += b2 * u2;
-        return result / sumbeta;
+        return o.div(result, sumbeta);
 #endif
     } else if constexpr (FAM == FAM_WENOZ) {
         // weno5_Z: omega_k = gamma_k (1 + (tau / (beta_k + eps))^2), eps = 1e-40.
@@ -576,13 +731,13 @@ CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, doub
         smoothness3(q0, q1, q2, q3, q4, b0, b1, b2);
         candidates3(q0, q1, q2, q3, q4, u0, u1, u2);
         double tau = fabs(b2 - b0), x;
-        x = tau / (b0 + eps); b0 = (1.0 / 16.0) * (1.0 + x * x);
-        x = tau / (b1 + eps); b1 = (5.0 / 8.0) * (1.0 + x * x);
-        x = tau / (b2 + eps); b2 = (5.0 / 16.0) * (1.0 + x * x);
-        double sumbeta = 0.0, result = 0.0;
-        sumbeta += b0; sumbeta += b1; sumbeta += b2;
+        x = o.div(tau, b0 + eps); b0 = (1.0 / 16.0) * (1.0 + x * x);
+        x = o.div(tau, b1 + eps); b1 = (5.0 / 8.0) * (1.0 + x * x);
+        x = o.div(tau, b2 + eps); b2 = (5.0 / 16.0) * (1.0 + x * x);
+        double sumbeta = b0, result = 0.0;  // 0 + b0 = b0 (b0 > 0)
+        sumbeta += b1; sumbeta += b2;
         result += b0 * u0; result += b1 * u1; result += b2 * u2;
-        return result / sumbeta;
+        return o.div(result, sumbeta);
     } else if constexpr (FAM == FAM_TENOZ) {
         // TENO5 with the Z-type measure (1 + tau/(beta_k + eps))^6 and the
         // cutoff measure_k < c * sum_j measure_j (Teno5_Z: interScheme.hpp:384-452).
@@ -630,79 +785,70 @@ CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, doub
         return q2 + delta * 0.5;
     }
 }
+template <int FAM>
+CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, double c, double kap = 0.0)
+{
+    OpsIeee o;
+    return inter5<FAM>(q0, q1, q2, q3, q4, c, kap, o);
+}
 
 // ---------------------------------------------------------------------------
 // cons -> prim as Equation::consToPrimEuler{1D,2D} (equation.cpp:37-93); the
 // 3D form adds w the same way.
 // ---------------------------------------------------------------------------
-template <int NV>
-CFD_HD void cons_to_prim(const double *c, double *p)
+// Returns 1/rho as the policy forms it (RN(1/rho) in the strict flavour).
+template <int NV, class O>
+CFD_HD double cons_to_prim(const double *c, double *p, O &o)
 {
     const double gamma = kGamma;
     if constexpr (NV == 3) {
         double r = c[0], ru = c[1], rE = c[2];
-#if defined(CFD_FAST)
-        const double ir = 1.0 / r;
-        double u = ru * ir;
-        double E = rE * ir;
-#else
-        const double ir = rcp_rn(r);
-        const double a[2] = {ru, rE}, bb[2] = {r, r}, yy[2] = {ir, ir};
-        double qq[2];
-        divs_rn<2>(a, bb, yy, qq);
-        double u = qq[0], E = qq[1];
-#endif
+        const double ir = o.rcp(r);
+        double u = o.div_y(ru, r, ir);
+        double E = o.div_y(rE, r, ir);
         double e = -u * u / 2 + E;
         double RT = (gamma - 1) * e;
         p[0] = r; p[1] = u; p[2] = r * RT;
+        return ir;
     } else if constexpr (NV == 4) {
         double r = c[0], ru = c[1], rv = c[2], rE = c[3];
-#if defined(CFD_FAST)
-        const double ir = 1.0 / r;
-        double u = ru * ir, v = rv * ir, E = rE * ir;
-#else
-        const double ir = rcp_rn(r);
-        const double a[3] = {ru, rv, rE}, bb[3] = {r, r, r}, yy[3] = {ir, ir, ir};
-        double qq[3];
-        divs_rn<3>(a, bb, yy, qq);
-        double u = qq[0], v = qq[1], E = qq[2];
-#endif
+        const double ir = o.rcp(r);
+        double u = o.div_y(ru, r, ir), v = o.div_y(rv, r, ir), E = o.div_y(rE, r, ir);
         double q2 = (u * u + v * v) / 2;
         double e = -q2 + E;
         double RT = (gamma - 1) * e;
         p[0] = r; p[1] = u; p[2] = v; p[3] = r * RT;
+        return ir;
     } else {
         double r = c[0], ru = c[1], rv = c[2], rw = c[3], rE = c[4];
-#if defined(CFD_FAST)
-        const double ir = 1.0 / r;
-        double u = ru * ir, v = rv * ir, w = rw * ir, E = rE * ir;
-#else
-        const double ir = rcp_rn(r);
-        const double a[4] = {ru, rv, rw, rE}, bb[4] = {r, r, r, r}, yy[4] = {ir, ir, ir, ir};
-        double qq[4];
-        divs_rn<4>(a, bb, yy, qq);
-        double u = qq[0], v = qq[1], w = qq[2], E = qq[3];
-#endif
+        const double ir = o.rcp(r);
+        double u = o.div_y(ru, r, ir), v = o.div_y(rv, r, ir), w = o.div_y(rw, r, ir), E = o.div_y(rE, r, ir);
         double q2 = (u * u + v * v + w * w) / 2;
         double e = -q2 + E;
         double RT = (gamma - 1) * e;
         p[0] = r; p[1] = u; p[2] = v; p[3] = w; p[4] = r * RT;
+        return ir;
     }
+}
+template <int NV>
+CFD_HD void cons_to_prim(const double *c, double *p)
+{
+    OpsIeee o;
+    cons_to_prim<NV>(c, p, o);
 }
 
 // prim -> cons as the eigensystem's primToCons/primToChar prologue
 // (eigenSystem.cpp:91-93 for 2D, :254-256 for 1D).
-template <int NV>
-CFD_HD void prim_to_cons(const double *p, double *c)
+template <int NV, class O>
+CFD_HD void prim_to_cons(const double *p, double *c, O &o)
 {
-    const double gamma = kGamma;
     if constexpr (NV == 3) {
         double rt = p[0], ut = p[1], pt = p[2];
         double ekt = (ut * ut) / 2;
 #if defined(CFD_FAST)
         c[0] = rt; c[1] = rt * ut; c[2] = pt * kInvGm1 + rt * ekt;
 #else
-        c[0] = rt; c[1] = rt * ut; c[2] = div_rn(pt, kGm1, kRcpGm1) + rt * ekt;
+        c[0] = rt; c[1] = rt * ut; c[2] = o.div_y(pt, kGm1, kRcpGm1) + rt * ekt;
 #endif
     } else if constexpr (NV == 4) {
         double rt = p[0], ut = p[1], vt = p[2], pt = p[3];
@@ -710,7 +856,7 @@ CFD_HD void prim_to_cons(const double *p, double *c)
 #if defined(CFD_FAST)
         c[0] = rt; c[1] = rt * ut; c[2] = rt * vt; c[3] = pt * kInvGm1 + rt * ekt;
 #else
-        c[0] = rt; c[1] = rt * ut; c[2] = rt * vt; c[3] = div_rn(pt, kGm1, kRcpGm1) + rt * ekt;
+        c[0] = rt; c[1] = rt * ut; c[2] = rt * vt; c[3] = o.div_y(pt, kGm1, kRcpGm1) + rt * ekt;
 #endif
     } else {
         double rt = p[0], ut = p[1], vt = p[2], wt = p[3], pt = p[4];
@@ -718,9 +864,16 @@ CFD_HD void prim_to_cons(const double *p, double *c)
 #if defined(CFD_FAST)
         c[0] = rt; c[1] = rt * ut; c[2] = rt * vt; c[3] = rt * wt; c[4] = pt * kInvGm1 + rt * ekt;
 #else
-        c[0] = rt; c[1] = rt * ut; c[2] = rt * vt; c[3] = rt * wt; c[4] = div_rn(pt, kGm1, kRcpGm1) + rt * ekt;
+        c[0] = rt; c[1] = rt * ut; c[2] = rt * vt; c[3] = rt * wt; c[4] = o.div_y(pt, kGm1, kRcpGm1) + rt * ekt;
 #endif
     }
+    (void)o;
+}
+template <int NV>
+CFD_HD void prim_to_cons(const double *p, double *c)
+{
+    OpsIeee o;
+    prim_to_cons<NV>(p, c, o);
 }
 
 // ---------------------------------------------------------------------------
@@ -738,29 +891,50 @@ struct Eigen {
 
     CFD_HD Eigen(const double *pl, const double *pr)
     {
+        OpsIeee o;
+        init(pl, pr, o);
+    }
+    template <class O>
+    CFD_HD Eigen(const double *pl, const double *pr, O &o)
+    {
+        init(pl, pr, o);
+    }
+
+  private:
+    template <class O>
+    CFD_HD void init(const double *pl, const double *pr, O &o)
+    {
         const double gamma = kGamma;
         if constexpr (NV == 3) {
             double rl = pl[0], ul = pl[1], pL = pl[2];
             double rr = pr[0], ur = pr[1], pR = pr[2];
 #if defined(CFD_FAST)
-            double HL = 0.5 * (ul * ul) + pL * (kG1 / rl);
-            double HR = 0.5 * (ur * ur) + pR * (kG1 / rr);
+            double HL = 0.5 * (ul * ul) + pL * o.div(kG1, rl);
+            double HR = 0.5 * (ur * ur) + pR * o.div(kG1, rr);
 #else
-            double HL = (ul * ul) / 2 + pL / rl * gamma / (gamma - 1);
-            double HR = (ur * ur) / 2 + pR / rr * gamma / (gamma - 1);
+            double HL = (ul * ul) / 2 + o.div_y(o.div(pL, rl) * gamma, kGm1, kRcpGm1);
+            double HR = (ur * ur) / 2 + o.div_y(o.div(pR, rr) * gamma, kGm1, kRcpGm1);
 #endif
-            double coef1 = sqrt(rl), coef2 = sqrt(rr);
-            double divisor = 1.0 / (coef1 + coef2);
+            double coef1 = o.sqrt(rl), coef2 = o.sqrt(rr);
+            double divisor = o.rcp(coef1 + coef2);
             double u = (coef1 * ul + coef2 * ur) * divisor;
             double ht = (coef1 * HL + coef2 * HR) * divisor;
             double ek = (u * u) / 2;
             double h = ht - ek;
-            double c = sqrt((gamma - 1) * h);
+            double c = o.sqrt((gamma - 1) * h);
             double g1 = gamma - 1;
-            double le[9] = {ht + c * (u - c) / g1, -u - c / g1, 1.0,
-                            -2.0 * ht + 4.0 * c * c / g1, 2.0 * u, -2.0,
-                            ht - c * (u + c) / g1, -u + c / g1, 1.0};
-            double f = 0.5 * g1 / (c * c);
+#if defined(CFD_FAST)
+            const double cg = o.spec ? c * kInvGm1 : c / g1;
+            double le[9] = {ht + (o.spec ? c * (u - c) * kInvGm1 : c * (u - c) / g1), -u - cg, 1.0,
+                            -2.0 * ht + (o.spec ? 4.0 * c * c * kInvGm1 : 4.0 * c * c / g1), 2.0 * u, -2.0,
+                            ht - (o.spec ? c * (u + c) * kInvGm1 : c * (u + c) / g1), -u + cg, 1.0};
+#else
+            const double cg = o.div_y(c, kGm1, kRcpGm1);
+            double le[9] = {ht + o.div_y(c * (u - c), kGm1, kRcpGm1), -u - cg, 1.0,
+                            -2.0 * ht + o.div_y(4.0 * c * c, kGm1, kRcpGm1), 2.0 * u, -2.0,
+                            ht - o.div_y(c * (u + c), kGm1, kRcpGm1), -u + cg, 1.0};
+#endif
+            double f = o.div_pos(0.5 * g1, c * c);
             for (int i = 0; i < 9; i++) L[i / 3][i % 3] = le[i] * f;
             double re[9] = {1.0, 1.0, 1.0, u - c, u, u + c, ht - u * c, 0.5 * u * u, ht + u * c};
             for (int i = 0; i < 9; i++) R[i / 3][i % 3] = re[i];
@@ -872,6 +1046,7 @@ struct Eigen {
         }
     }
 
+  public:
     // char = L * cons with the reference's summation order
     // (1D: rt L0 + rut L1 + ret L2, eigenSystem.cpp:260-264;
     //  2D: rut L1 + rvt L2 + ret L3 + rt L0, eigenSystem.cpp:97-106;
@@ -906,48 +1081,48 @@ struct Eigen {
 };
 
 // charToPrim's cons -> prim tail (2D: eigenSystem.cpp:163-167; 3D adds w).
-template <int NV>
-CFD_HD void char_cons_to_prim(const double *cs, double *p)
+// Returns 1/rho as the policy forms it.
+template <int NV, class O>
+CFD_HD double char_cons_to_prim(const double *cs, double *p, O &o)
 {
     const double gamma = kGamma;
     if constexpr (NV == 3) {
         // eigensystemEuler1D::consToPrim (eigenSystem.cpp:309-322)
         double rt = cs[0], rut = cs[1], ret = cs[2];
-        double ut = rut / rt;
+        const double irt = o.spec ? o.rcp(rt) : 0.0;
+        double ut = o.spec ? o.div_y(rut, rt, irt) : rut / rt;
         double ekt = (ut * ut) / 2;  // one division only
         p[0] = rt; p[1] = ut; p[2] = (gamma - 1) * (ret - rt * ekt);
+        return irt;
     } else if constexpr (NV == 4) {
         double rt = cs[0], rut = cs[1], rvt = cs[2], ret = cs[3];
+        const double irt = o.rcp(rt);
+        double ut = o.div_y(rut, rt, irt), vt = o.div_y(rvt, rt, irt);
 #if defined(CFD_FAST)
-        const double irt = 1.0 / rt;
-        double ut = rut * irt, vt = rvt * irt;
         double rekt = (rut * rut + rvt * rvt) * (0.5 * irt);
 #else
-        const double irt = rcp_rn(rt);
-        const double a[3] = {rut, rvt, rut * rut + rvt * rvt}, bb[3] = {rt, rt, rt}, yy[3] = {irt, irt, irt};
-        double qq[3];
-        divs_rn<3>(a, bb, yy, qq);
-        double ut = qq[0], vt = qq[1];
-        double rekt = qq[2] / 2;
+        double rekt = o.div_y(rut * rut + rvt * rvt, rt, irt) / 2;
 #endif
         p[0] = rt; p[1] = ut; p[2] = vt; p[3] = (gamma - 1) * (ret - rekt);
+        return irt;
     } else {
         double rt = cs[0], rut = cs[1], rvt = cs[2], rwt = cs[3], ret = cs[4];
+        const double irt = o.rcp(rt);
+        double ut = o.div_y(rut, rt, irt), vt = o.div_y(rvt, rt, irt), wt = o.div_y(rwt, rt, irt);
 #if defined(CFD_FAST)
-        const double irt = 1.0 / rt;
-        double ut = rut * irt, vt = rvt * irt, wt = rwt * irt;
         double rekt = (rut * rut + rvt * rvt + rwt * rwt) * (0.5 * irt);
 #else
-        const double irt = rcp_rn(rt);
-        const double a[4] = {rut, rvt, rwt, rut * rut + rvt * rvt + rwt * rwt}, bb[4] = {rt, rt, rt, rt},
-                     yy[4] = {irt, irt, irt, irt};
-        double qq[4];
-        divs_rn<4>(a, bb, yy, qq);
-        double ut = qq[0], vt = qq[1], wt = qq[2];
-        double rekt = qq[3] / 2;
+        double rekt = o.div_y(rut * rut + rvt * rvt + rwt * rwt, rt, irt) / 2;
 #endif
         p[0] = rt; p[1] = ut; p[2] = vt; p[3] = wt; p[4] = (gamma - 1) * (ret - rekt);
+        return irt;
     }
+}
+template <int NV>
+CFD_HD void char_cons_to_prim(const double *cs, double *p)
+{
+    OpsIeee o;
+    char_cons_to_prim<NV>(cs, p, o);
 }
 
 // variable_positive_limiter (positive_preserving.hpp:13-46) applied to the
@@ -1010,28 +1185,46 @@ CFD_HD void positive_limit_md(int which, const double *W, double *Wi)
     for (int i = 0; i < NV; i++) Wi[i] = (1 - theta) * W[i] + theta * Wi[i];
 }
 
+// Whether the positivity limiters above leave the face state with cons c and
+// prim p alone, whatever the rounding of their own pressure: density and
+// gamma p at least 1e-10, gamma p by more than 1e-12 of the energy terms it
+// is the difference of.
+template <int NV>
+CFD_HD bool face_positive(const double *c, const double *p)
+{
+    return (c[0] >= 1e-10) & (kGamma * p[NV - 1] >= 1e-10 + 1e-12 * c[NV - 1]);
+}
+
 // ---------------------------------------------------------------------------
 // Face reconstruction (Recon5Order{1D,2D}EulerEig::reconI,
 // reconstructor5order.hpp:233-323 and 326-429). cs6/pr6 are the re-derived
 // cons and the prim of the six stencil cells (face between cell 2 and 3).
 // Writes the left and right face prim states.
 // ---------------------------------------------------------------------------
-template <int NV, int AX, int FAM>
+// ir: 1/rho of both states (speculative policies).
+template <int NV, int AX, int FAM, class O>
 CFD_HD void reconstruct_face(const double (*pr6)[NV], const double (*cs6)[NV], double icst, double kap,
-                             double *fl, double *fr)
+                             double *fl, double *fr, O &o, double *ir)
 {
-    Eigen<NV, AX> eig(pr6[2], pr6[3]);
+    Eigen<NV, AX> eig(pr6[2], pr6[3], o);
     double QL[NV], QR[NV];
     for (int k = 0; k < NV; k++) {
         double q[6];
         for (int j = 0; j < 6; j++) q[j] = eig.project(k, cs6[j]);
-        QL[k] = inter5<FAM>(q[0], q[1], q[2], q[3], q[4], icst, kap);
-        QR[k] = inter5<FAM>(q[5], q[4], q[3], q[2], q[1], icst, kap);
+        QL[k] = inter5<FAM>(q[0], q[1], q[2], q[3], q[4], icst, kap, o);
+        QR[k] = inter5<FAM>(q[5], q[4], q[3], q[2], q[1], icst, kap, o);
     }
     double cl[NV], cr[NV];
     eig.back(QL, cl);
     eig.back(QR, cr);
-    if constexpr (NV == 3) {
+    if constexpr (NV == 3 && O::spec) {
+        // the limiter acts on a density or a gamma p below its 1e-10: with both
+        // clearly above it leaves the state alone
+        ir[0] = char_cons_to_prim<3>(cl, fl, o);
+        ir[1] = char_cons_to_prim<3>(cr, fr, o);
+        o.need(face_positive<3>(cl, fl));
+        o.need(face_positive<3>(cr, fr));
+    } else if constexpr (NV == 3) {
         double consL[3], consR[3];
         prim_to_cons<3>(pr6[2], consL);
         prim_to_cons<3>(pr6[3], consR);
@@ -1055,6 +1248,15 @@ CFD_HD void reconstruct_face(const double (*pr6)[NV], const double (*cs6)[NV], d
             fr[NV - 1] = pr6[3][NV - 1];
         }
     }
+    (void)ir;
+}
+template <int NV, int AX, int FAM>
+CFD_HD void reconstruct_face(const double (*pr6)[NV], const double (*cs6)[NV], double icst, double kap,
+                             double *fl, double *fr)
+{
+    OpsIeee o;
+    double ir[2];
+    reconstruct_face<NV, AX, FAM>(pr6, cs6, icst, kap, fl, fr, o, ir);
 }
 
 // ---------------------------------------------------------------------------
@@ -1089,10 +1291,12 @@ struct EigenBase {
         }
         roe_weights(pl, kl);
         roe_weights(prr, kr);
-        init(kl, kr);
+        OpsIeee o;
+        init(kl, kr, o);
     }
     // from the two cells' Roe weights (roe_weights), e.g. kept per cell by the sweep
-    CFD_HD EigenBase(const double *kl, const double *kr) { init(kl, kr); }
+    template <class O>
+    CFD_HD EigenBase(const double *kl, const double *kr, O &o) { init(kl, kr, o); }
 
     // A cell's share of the Roe average: (sqrt(rho), sqrt(rho) u, sqrt(rho) v,
     // [sqrt(rho) w,] sqrt(rho) H), each product rounded as the reference's
@@ -1100,19 +1304,27 @@ struct EigenBase {
     // p / rho * gamma / (gamma - 1).
     static CFD_HD void roe_weights(const double *p, double *k)
     {
+        OpsIeee o;
+        roe_weights(p, k, o.rcp(p[0]), o);
+    }
+    // ir: 1/rho as the policy forms it
+    template <class O>
+    static CFD_HD void roe_weights(const double *p, double *k, double irho, O &o)
+    {
         constexpr int D = NV - 2, E = NV - 1;
+        (void)irho;
         const double r = p[0], pp = p[E];
         double q2 = p[1] * p[1] + p[2] * p[2];
         if constexpr (D == 3) q2 = q2 + p[3] * p[3];
 #if defined(CFD_FAST)
         // sqrt(rho) = rho rsqrt(rho), sqrt(rho) H = sqrt(rho) |v|^2 / 2 +
         // gamma/(gamma-1) p rsqrt(rho)
-        const double ir = rsqrt(r);
+        const double ir = o.rsqrt(r);
         const double coef = r * ir;
         k[E] = 0.5 * (coef * q2) + kG1 * (pp * ir);
 #else
-        const double coef = sqrt(r);
-        const double H = q2 / 2 + div_rn(pp / r * kGamma, kGm1, kRcpGm1);
+        const double coef = o.sqrt(r);
+        const double H = q2 / 2 + o.div_y(o.div_y(pp, r, irho) * kGamma, kGm1, kRcpGm1);
         k[E] = coef * H;
 #endif
         k[0] = coef;
@@ -1121,11 +1333,12 @@ struct EigenBase {
     }
 
   private:
-    CFD_HD void init(const double *kl, const double *kr)
+    template <class O>
+    CFD_HD void init(const double *kl, const double *kr, O &o)
     {
         constexpr int D = NV - 2;
         const double gamma = kGamma;
-        const double divisor = 1.0 / (kl[0] + kr[0]);
+        const double divisor = o.rcp(kl[0] + kr[0]);
         u = (kl[1] + kr[1]) * divisor;
         v = (kl[2] + kr[2]) * divisor;
         w = (D == 3) ? (kl[3] + kr[3]) * divisor : 0.0;
@@ -1141,25 +1354,18 @@ struct EigenBase {
 #if defined(CFD_FAST)
         // 1/c = rsqrt(c^2), 1/h = (gamma - 1) / c^2
         const double c2 = (gamma - 1) * h;
-        ic = rsqrt(c2);
+        ic = o.rsqrt(c2);
         c = c2 * ic;
         ih = (gamma - 1) * (ic * ic);
 #else
-        c = sqrt((gamma - 1) * h);
-        ic = rcp_rn(c);
-        ih = rcp_rn(h);
-        if constexpr (D == 2) {
-            const double a[4] = {Vn, ek, u, v}, bb[4] = {c, h, h, h}, yy[4] = {ic, ih, ih, ih};
-            double qq[4];
-            divs_rn<4>(a, bb, yy, qq);
-            Vc = qq[0]; ekh = qq[1]; uh = qq[2]; vh = qq[3];
-            wh = 0.0;
-        } else {
-            const double a[5] = {Vn, ek, u, v, w}, bb[5] = {c, h, h, h, h}, yy[5] = {ic, ih, ih, ih, ih};
-            double qq[5];
-            divs_rn<5>(a, bb, yy, qq);
-            Vc = qq[0]; ekh = qq[1]; uh = qq[2]; vh = qq[3]; wh = qq[4];
-        }
+        c = o.sqrt((gamma - 1) * h);
+        ic = o.rcp(c);
+        ih = o.rcp(h);
+        Vc = o.div_y(Vn, c, ic);
+        ekh = o.div_y(ek, h, ih);
+        uh = o.div_y(u, h, ih);
+        vh = o.div_y(v, h, ih);
+        wh = (D == 3) ? o.div_y(w, h, ih) : 0.0;
 #endif
     }
 
@@ -1232,9 +1438,10 @@ struct EigenBase {
 // cs(j, v): re-derived cons of stencil cell j (0..5), pr(j, v): its prim;
 // eb: the face's Roe-averaged eigensystem; posl: the positivity option
 // (cfd_config.positivity) instead of the reference's fallback.
-template <int NV, int AX, int FAM, class CS, class PR>
+// ir: 1/rho of both states (speculative policies).
+template <int NV, int AX, int FAM, class CS, class PR, class O>
 CFD_HD void reconstruct_face_stream(const EigenBase<NV, AX> &eb, const CS &cs, const PR &pr, double icst, double kap,
-                                    double *fl, double *fr, int posl = 0)
+                                    double *fl, double *fr, int posl, O &o, double *ir)
 {
     static_assert(NV == 4 || NV == 5, "multi-dimensional form");
     double cl[NV], cr[NV];
@@ -1262,15 +1469,15 @@ CFD_HD void reconstruct_face_stream(const EigenBase<NV, AX> &eb, const CS &cs, c
         }
         double QL, QR;
 #if !defined(CFD_ROLL_FIELDS)
-        QL = inter5<FAM>(q[0], q[1], q[2], q[3], q[4], icst, kap);
-        QR = inter5<FAM>(q[5], q[4], q[3], q[2], q[1], icst, kap);
+        QL = inter5<FAM>(q[0], q[1], q[2], q[3], q[4], icst, kap, o);
+        QR = inter5<FAM>(q[5], q[4], q[3], q[2], q[1], icst, kap, o);
 #else
         // one interpolator body for both states (mirrored stencil on side 1)
 #pragma unroll 1
         for (int side = 0; side < 2; side++) {
             const bool m = side != 0;
             const double r = inter5<FAM>(m ? q[5] : q[0], m ? q[4] : q[1], q[m ? 3 : 2], q[m ? 2 : 3],
-                                         m ? q[1] : q[4], icst, kap);
+                                         m ? q[1] : q[4], icst, kap, o);
             if (m) QR = r; else QL = r;
         }
 #endif
@@ -1286,6 +1493,15 @@ CFD_HD void reconstruct_face_stream(const EigenBase<NV, AX> &eb, const CS &cs, c
             }
         }
     }
+    if constexpr (O::spec) {
+        // neither the reference's fallback nor the positivity option may act
+        ir[0] = char_cons_to_prim<NV>(cl, fl, o);
+        ir[1] = char_cons_to_prim<NV>(cr, fr, o);
+        o.need(!(fl[0] < 0 || fl[NV - 1] < 0) & !(fr[0] < 0 || fr[NV - 1] < 0));
+        if (posl) o.need(face_positive<NV>(cl, fl) & face_positive<NV>(cr, fr));
+        return;
+    }
+    (void)ir;
     if (posl) {
         // the 1D char-recon limiter (reconstructor5order.hpp:225-236): density
         // of both states, then gamma p of both, against the cells' cons
@@ -1299,12 +1515,12 @@ CFD_HD void reconstruct_face_stream(const EigenBase<NV, AX> &eb, const CS &cs, c
         positive_limit_md<NV>(0, WR, cr);
         positive_limit_md<NV>(1, WL, cl);
         positive_limit_md<NV>(1, WR, cr);
-        char_cons_to_prim<NV>(cl, fl);
-        char_cons_to_prim<NV>(cr, fr);
+        char_cons_to_prim<NV>(cl, fl, o);
+        char_cons_to_prim<NV>(cr, fr, o);
         return;
     }
-    char_cons_to_prim<NV>(cl, fl);
-    char_cons_to_prim<NV>(cr, fr);
+    char_cons_to_prim<NV>(cl, fl, o);
+    char_cons_to_prim<NV>(cr, fr, o);
     // crude positivity fallback (reconstructor5order.hpp:380-381), including
     // the reference's mix of right density/pressure with left velocity.
     if (fl[0] < 0 || fl[NV - 1] < 0) {
@@ -1323,7 +1539,8 @@ CFD_HD void reconstruct_face_stream(const CS &cs, const PR &pr, double icst, dou
                                     int posl = 0)
 {
     const EigenBase<NV, AX> eb(pr);
-    reconstruct_face_stream<NV, AX, FAM>(eb, cs, pr, icst, kap, fl, fr, posl);
+    OpsIeee o;
+    reconstruct_face_stream<NV, AX, FAM>(eb, cs, pr, icst, kap, fl, fr, posl, o, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1332,18 +1549,52 @@ CFD_HD void reconstruct_face_stream(const CS &cs, const PR &pr, double icst, dou
 enum FluxKind : int { FLUX_HLLC = 0, FLUX_ROE = 1 };
 
 // HLLCFlux1D (fluxSchemes.hpp:74-125)
-CFD_HD void hllc_1d(const double *L, const double *R, double *res)
+// (ir: 1/rho of both states, used by the speculative policies here and below)
+template <class O>
+CFD_HD void hllc_1d(const double *L, const double *R, double *res, O &o, const double *ir)
 {
     const double gamma = kGamma;
     double rl = L[0], ul = L[1], pl = L[2], rr = R[0], ur = R[1], pr = R[2];
-    double HL = pl / rl * kGamma / (kGamma - 1) + (ul * ul) / 2;
-    double HR = pr / rr * kGamma / (kGamma - 1) + (ur * ur) / 2;
-    double cl = sqrt(gamma * (pl / rl));
-    double cr = sqrt(gamma * (pr / rr));
+    double prl, prr, HL, HR;
+    if constexpr (O::spec) {
+        prl = o.div_y(pl, rl, ir[0]);
+        prr = o.div_y(pr, rr, ir[1]);
+        HL = o.div_y(prl * kGamma, kGm1, kRcpGm1) + (ul * ul) / 2;
+        HR = o.div_y(prr * kGamma, kGm1, kRcpGm1) + (ur * ur) / 2;
+    } else {
+        prl = pl / rl;
+        prr = pr / rr;
+        HL = pl / rl * kGamma / (kGamma - 1) + (ul * ul) / 2;
+        HR = pr / rr * kGamma / (kGamma - 1) + (ur * ur) / 2;
+    }
+    double cl = o.sqrt(gamma * prl);
+    double cr = o.sqrt(gamma * prr);
     // std::min(ur - cr, ul - cl) and std::max(ul + cl, ur + cr)
     double SL = ((ul - cl) < (ur - cr)) ? (ul - cl) : (ur - cr);
     double SR = ((ul + cl) < (ur + cr)) ? (ur + cr) : (ul + cl);
-    double Sstar = ((pr - pl) + (rl * ul * (SL - ul) - rr * ur * (SR - ur))) / (rl * (SL - ul) - rr * (SR - ur));
+    // the denominator is negative: (-a) / (-b) = a / b for the policies
+    double Sstar = o.div(-((pr - pl) + (rl * ul * (SL - ul) - rr * ur * (SR - ur))), -(rl * (SL - ul) - rr * (SR - ur)));
+    if constexpr (O::spec) {
+        // one side's star flux, selected by value; the supersonic sides keep F
+        const bool left = SL >= 0 || Sstar >= 0, star = left ? !(SL >= 0) : SR >= 0;
+        const double r = left ? rl : rr, u = left ? ul : ur, p = left ? pl : pr, H = left ? HL : HR,
+                     S = left ? SL : SR;
+        const double F[3] = {r * u, r * u * u + p, r * H * u};
+        const double U[3] = {r, r * u, o.div_y(p, kGm1, kRcpGm1) + r * u * u / 2};
+        const double pStar = p + r * (S - u) * (Sstar - u);
+        const double D[3] = {0, 1, Sstar};
+        // S - S* is negative on the left, positive on the right
+        const double d = left ? -(S - Sstar) : S - Sstar;
+        o.need(!star | O::in_range(d));
+        const double y = O::rcp_near(d);
+        for (int i = 0; i < 3; i++) {
+            const double a = Sstar * (S * U[i] - F[i]) + S * pStar * D[i];
+            const double as = left ? -a : a;
+            o.need(!star | O::in_range_or_0(as));
+            res[i] = star ? O::quot(as, d, y) : F[i];
+        }
+        return;
+    }
     if (SL >= 0) {
         res[0] = rl * ul; res[1] = rl * ul * ul + pl; res[2] = rl * HL * ul;
     } else if (Sstar >= 0) {
@@ -1364,26 +1615,33 @@ CFD_HD void hllc_1d(const double *L, const double *R, double *res)
 }
 
 // roeFlux1D2 (fluxSchemes.hpp:13-71)
-CFD_HD void roe_1d(const double *L, const double *R, double *res)
+template <class O>
+CFD_HD void roe_1d(const double *L, const double *R, double *res, O &o, const double *ir)
 {
     const double gamma = kGamma;
     double rl = L[0], ul = L[1], pl = L[2], rr = R[0], ur = R[1], pr = R[2];
-    double HL = pl / rl * kGamma / (kGamma - 1) + (ul * ul) / 2;
-    double HR = pr / rr * kGamma / (kGamma - 1) + (ur * ur) / 2;
-    double srl = sqrt(rl), srr = sqrt(rr);
-    double rBar = sqrt(rl * rr);
-    double uBar = (ul * srl + ur * srr) / (srl + srr);
-    double HBar = (HL * srl + HR * srr) / (srl + srr);
-    double cBar = sqrt((gamma - 1) * (HBar - uBar * uBar / 2));
+    double HL, HR;
+    if constexpr (O::spec) {
+        HL = o.div_y(o.div_y(pl, rl, ir[0]) * kGamma, kGm1, kRcpGm1) + (ul * ul) / 2;
+        HR = o.div_y(o.div_y(pr, rr, ir[1]) * kGamma, kGm1, kRcpGm1) + (ur * ur) / 2;
+    } else {
+        HL = pl / rl * kGamma / (kGamma - 1) + (ul * ul) / 2;
+        HR = pr / rr * kGamma / (kGamma - 1) + (ur * ur) / 2;
+    }
+    double srl = o.sqrt(rl), srr = o.sqrt(rr);
+    double rBar = o.sqrt(rl * rr);
+    double uBar = o.div(ul * srl + ur * srr, srl + srr);
+    double HBar = o.div(HL * srl + HR * srr, srl + srr);
+    double cBar = o.sqrt((gamma - 1) * (HBar - uBar * uBar / 2));
     double cBar2 = (gamma - 1) * (HBar - uBar * uBar / 2);
     double dr = rr - rl, du = ur - ul, dp = pr - pl;
     double lambda[3] = {fabs(uBar), fabs(uBar + cBar), fabs(uBar - cBar)};
     double eps = 0.1 * (fabs(uBar) + cBar);
     for (int i = 0; i < 3; i++)
-        if (lambda[i] < eps) lambda[i] = (lambda[i] * lambda[i] + eps * eps) / (2.0 * eps);
-    double a0 = lambda[0] * (dr - dp / cBar2);
-    double a1 = lambda[1] / (2.0 * cBar2) * (dp + rBar * cBar * du);
-    double a2 = lambda[2] / (2.0 * cBar2) * (dp - rBar * cBar * du);
+        if (lambda[i] < eps) lambda[i] = o.div(lambda[i] * lambda[i] + eps * eps, 2.0 * eps);
+    double a0 = lambda[0] * (dr - o.div(dp, cBar2));
+    double a1 = o.div(lambda[1], 2.0 * cBar2) * (dp + rBar * cBar * du);
+    double a2 = o.div(lambda[2], 2.0 * cBar2) * (dp - rBar * cBar * du);
     double a3 = a0 + a1 + a2;
     double a4 = cBar * (a1 - a2);
     double FL[3] = {rl * ul, rl * ul * ul + pl, rl * HL * ul};
@@ -1391,13 +1649,13 @@ CFD_HD void roe_1d(const double *L, const double *R, double *res)
     for (int i = 0; i < 3; i++) res[i] = (FL[i] + FR[i]) / 2.0;
     res[0] -= 0.5 * a3;
     res[1] -= 0.5 * (a3 * uBar + a4);
-    res[2] -= 0.5 * (HBar * a3 + uBar * a4 - cBar2 * a0 / (gamma - 1));
+    res[2] -= 0.5 * (HBar * a3 + uBar * a4 - (O::spec ? o.div_y(cBar2 * a0, kGm1, kRcpGm1) : cBar2 * a0 / (gamma - 1)));
 }
 
 // HLLCFlux2D2 (fluxSchemes.hpp:202-327); the 3D form treats the two
 // tangential momentum components alike.
-template <int NV, int AX>
-CFD_HD void hllc_md(const double *L, const double *R, double *res)
+template <int NV, int AX, class O>
+CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const double *ir)
 {
     constexpr int D = NV - 2, E = NV - 1;
     const double gamma = kGamma;
@@ -1406,7 +1664,7 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res)
     const double *vl = L + 1, *vr = R + 1;
     double HL, HR;
 #if defined(CFD_FAST)
-    const double prl = pl * (1.0 / rl), prr = pr * (1.0 / rr);  // p / rho
+    const double prl = pl * (O::spec ? ir[0] : 1.0 / rl), prr = pr * (O::spec ? ir[1] : 1.0 / rr);  // p / rho
     {
         double kl = vl[0] * vl[0] + vl[1] * vl[1], kr = vr[0] * vr[0] + vr[1] * vr[1];
         if constexpr (D == 3) { kl += vl[2] * vl[2]; kr += vr[2] * vr[2]; }
@@ -1414,14 +1672,12 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res)
         HR = 0.5 * kr + prr * kG1;
     }
     double VnL = vl[AX], VnR = vr[AX];
-    double cl = sqrt(prl * gamma), cr = sqrt(prr * gamma);
+    double cl = o.sqrt(prl * gamma), cr = o.sqrt(prr * gamma);
 #else
-    const double prl = pl / rl, prr = pr / rr;
-    // x / (gamma - 1) by its correctly rounded reciprocal (divs_rn)
+    const double prl = O::spec ? o.div_y(pl, rl, ir[0]) : pl / rl, prr = O::spec ? o.div_y(pr, rr, ir[1]) : pr / rr;
+    // x / (gamma - 1) by its correctly rounded reciprocal
     {
-        const double a[2] = {prl * kGamma, prr * kGamma}, bb[2] = {kGm1, kGm1}, yy[2] = {kRcpGm1, kRcpGm1};
-        double qq[2];
-        divs_rn<2>(a, bb, yy, qq);
+        const double qq[2] = {o.div_y(prl * kGamma, kGm1, kRcpGm1), o.div_y(prr * kGamma, kGm1, kRcpGm1)};
         if constexpr (D == 2) {
             HL = (vl[0] * vl[0] + vl[1] * vl[1]) / 2 + qq[0];
             HR = (vr[0] * vr[0] + vr[1] * vr[1]) / 2 + qq[1];
@@ -1431,21 +1687,33 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res)
         }
     }
     double VnL = vl[AX], VnR = vr[AX];
-    double cl = sqrt(prl * gamma), cr = sqrt(prr * gamma);
+    double cl = o.sqrt(prl * gamma), cr = o.sqrt(prr * gamma);
 #endif
+    (void)ir;
     double rBar = (rl + rr) / 2, cBar = (cl + cr) / 2;
     double ps0 = (pl + pr) / 2 - rBar * cBar * (VnR - VnL) / 2;
     double ps = (0.0 < ps0) ? ps0 : 0.0;  // std::max(0.0, .)
-    double ql = (ps <= pl) ? 1.0 : sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (ps / pl - 1.0));
-    double qr = (ps <= pr) ? 1.0 : sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (ps / pr - 1.0));
+    double ql, qr;
+    if constexpr (O::spec) {
+        const double tl = o.sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (o.div(ps, pl) - 1.0));
+        const double tr = o.sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (o.div(ps, pr) - 1.0));
+        ql = (ps <= pl) ? 1.0 : tl;
+        qr = (ps <= pr) ? 1.0 : tr;
+    } else {
+        ql = (ps <= pl) ? 1.0 : sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (ps / pl - 1.0));
+        qr = (ps <= pr) ? 1.0 : sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (ps / pr - 1.0));
+    }
     double SL = VnL - cl * ql, SR = VnR + cr * qr;
-    double Sstar = ((pr - pl) + (rl * VnL * (SL - VnL) - rr * VnR * (SR - VnR))) / (rl * (SL - VnL) - rr * (SR - VnR));
+    // the denominator is negative: (-a) / (-b) = a / b for the policies
+    double Sstar = o.div(-((pr - pl) + (rl * VnL * (SL - VnL) - rr * VnR * (SR - VnR))),
+                         -(rl * (SL - VnL) - rr * (SR - VnR)));
 
     // Physical flux F and star-state difference for one side
     // (the reference spells the tangential selector as u*norm[1] / v*norm[0];
     // for unit axis normals that is u_i * (1 - n_i)).
+    // neg: S - Vn and S - S* are negative (the left side)
     auto side_flux = [&](double r, const double *v, double p, double H, double Vn, double S, double *out, double scale,
-                         bool accumulate) {
+                         bool accumulate, bool neg) {
         double U[NV], F[NV], Ustar[NV];
         U[0] = r;
         for (int i = 0; i < D; i++) U[1 + i] = r * v[i];
@@ -1453,10 +1721,12 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res)
         F[0] = r * Vn;
         for (int i = 0; i < D; i++) F[1 + i] = r * v[i] * Vn + p * n[i];
         F[E] = r * H * Vn;
-        double Usf = (S - Vn) / (S - Sstar);
+        const double SV = neg ? -(S - Vn) : S - Vn, SS = neg ? -(S - Sstar) : S - Sstar;
+        double Usf = O::spec ? o.div(SV, SS) : (S - Vn) / (S - Sstar);
+        const double pS = O::spec ? o.div(neg ? -p : p, SV) : p / (S - Vn);
         Ustar[0] = Usf * r;
         for (int i = 0; i < D; i++) Ustar[1 + i] = Usf * (Sstar * n[i] + v[i] * (1.0 - n[i])) * r;
-        Ustar[E] = Usf * (U[E] + (Sstar - Vn) * (r * Sstar + p / (S - Vn)));
+        Ustar[E] = Usf * (U[E] + (Sstar - Vn) * (r * Sstar + pS));
         for (int i = 0; i < NV; i++) {
             double f = F[i] + S * (Ustar[i] - U[i]);
             f = (scale != 1.0) ? f / 2 : f;
@@ -1481,7 +1751,7 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res)
 #pragma unroll
             for (int i = 0; i < D; i++) vs[i] = useL ? vl[i] : vr[i];
             side_flux(useL ? rl : rr, vs, useL ? pl : pr, useL ? HL : HR, useL ? VnL : VnR, useL ? SL : SR, res,
-                      avg ? 0.5 : 1.0, it > 0);
+                      avg ? 0.5 : 1.0, it > 0, useL);
         }
     } else {
         res[0] = rr * VnR;
@@ -1495,8 +1765,8 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res)
 // roots: sqrt(rho) = rho rsqrt(rho), sqrt(rho) H = sqrt(rho) |v|^2 / 2 +
 // gamma/(gamma-1) p rsqrt(rho), rho H = rho |v|^2 / 2 + gamma/(gamma-1) p,
 // 1/c = rsqrt(c^2); the entropy fix's 1/(2 eps) only where a wave needs it.
-template <int NV, int AX>
-CFD_HD void roe_md_fast(const double *L, const double *R, double *res)
+template <int NV, int AX, class O>
+CFD_HD void roe_md_fast(const double *L, const double *R, double *res, O &o)
 {
     constexpr int D = NV - 2, E = NV - 1;
     const double n[3] = {AX == 0 ? 1.0 : 0.0, AX == 1 ? 1.0 : 0.0, AX == 2 ? 1.0 : 0.0};
@@ -1510,9 +1780,9 @@ CFD_HD void roe_md_fast(const double *L, const double *R, double *res)
     for (int i = 0; i < D; i++) Fc[1 + i] = rl * vl[i] * VnL + rr * vr[i] * VnR + (pl + pr) * n[i];
     Fc[E] = (0.5 * rl * kl + kG1 * pl) * VnL + (0.5 * rr * kr + kG1 * pr) * VnR;
 
-    const double ir1 = rsqrt(rl), ir2 = rsqrt(rr);
+    const double ir1 = o.rsqrt(rl), ir2 = o.rsqrt(rr);
     const double coef1 = rl * ir1, coef2 = rr * ir2;
-    const double divisor = 1.0 / (coef1 + coef2);
+    const double divisor = o.rcp(coef1 + coef2);
     const double rhoAvg = coef1 * coef2;
     double vAvg[3];
     for (int i = 0; i < D; i++) vAvg[i] = (coef1 * vl[i] + coef2 * vr[i]) * divisor;
@@ -1521,13 +1791,13 @@ CFD_HD void roe_md_fast(const double *L, const double *R, double *res)
     if constexpr (D == 2) q_2Avg = (vAvg[0] * vAvg[0] + vAvg[1] * vAvg[1]) / 2;
     else q_2Avg = (vAvg[0] * vAvg[0] + vAvg[1] * vAvg[1] + vAvg[2] * vAvg[2]) / 2;
     const double c2 = (kGamma - 1) * (HAvg - q_2Avg);
-    const double ic = rsqrt(c2);
+    const double ic = o.rsqrt(c2);
     const double cAvg = c2 * ic, ic2 = ic * ic;
     const double VnAvg = vAvg[AX];
     double lambda[3] = {fabs(VnAvg - cAvg), fabs(VnAvg), fabs(VnAvg + cAvg)};
     const double eps = 0.05 * (fabs(VnAvg) + cAvg);
     if (lambda[0] < eps || lambda[1] < eps || lambda[2] < eps) {
-        const double ie2 = 0.5 / eps;
+        const double ie2 = o.div_pos(0.5, eps);
         for (int i = 0; i < 3; i++)
             if (lambda[i] < eps) lambda[i] = (lambda[i] * lambda[i] + eps * eps) * ie2;
     }
@@ -1571,22 +1841,22 @@ Lam3 entropy_fix3(double l0, double l1, double l2, double eps)
 
 // roeFlux2DSym (fluxSchemes.hpp:420-553), 3D form with both tangential
 // components in the linear wave.
-template <int NV, int AX>
-CFD_HD void roe_md(const double *L, const double *R, double *res)
+template <int NV, int AX, class O>
+CFD_HD void roe_md(const double *L, const double *R, double *res, O &o, const double *ir)
 {
 #if defined(CFD_FAST)
-    roe_md_fast<NV, AX>(L, R, res);
+    (void)ir;
+    roe_md_fast<NV, AX>(L, R, res, o);
 #else
     constexpr int D = NV - 2, E = NV - 1;
     const double n[3] = {AX == 0 ? 1.0 : 0.0, AX == 1 ? 1.0 : 0.0, AX == 2 ? 1.0 : 0.0};
     double rl = L[0], rr = R[0], pl = L[E], pr = R[E];
     const double *vl = L + 1, *vr = R + 1;
     double HL, HR;
-    // x / (gamma - 1) by its correctly rounded reciprocal (divs_rn)
+    // x / (gamma - 1) by its correctly rounded reciprocal
     {
-        const double a[2] = {pl / rl * kGamma, pr / rr * kGamma}, bb[2] = {kGm1, kGm1}, yy[2] = {kRcpGm1, kRcpGm1};
-        double qq[2];
-        divs_rn<2>(a, bb, yy, qq);
+        const double prl = O::spec ? o.div_y(pl, rl, ir[0]) : pl / rl, prr = O::spec ? o.div_y(pr, rr, ir[1]) : pr / rr;
+        const double qq[2] = {o.div_y(prl * kGamma, kGm1, kRcpGm1), o.div_y(prr * kGamma, kGm1, kRcpGm1)};
         if constexpr (D == 2) {
             HL = (vl[0] * vl[0] + vl[1] * vl[1]) / 2 + qq[0];
             HR = (vr[0] * vr[0] + vr[1] * vr[1]) / 2 + qq[1];
@@ -1604,24 +1874,32 @@ CFD_HD void roe_md(const double *L, const double *R, double *res)
     for (int i = 0; i < D; i++) FcR[1 + i] = rr * vr[i] * VnR + pr * n[i];
     FcR[E] = rr * HR * VnR;
 
-    double coef1 = sqrt(rl), coef2 = sqrt(rr);
-    double divisor = 1.0 / (coef1 + coef2);
-    double rhoAvg = sqrt(rl * rr);
+    double coef1 = o.sqrt(rl), coef2 = o.sqrt(rr);
+    double divisor = o.rcp(coef1 + coef2);
+    double rhoAvg = o.sqrt(rl * rr);
     double vAvg[3];
     for (int i = 0; i < D; i++) vAvg[i] = (coef1 * vl[i] + coef2 * vr[i]) * divisor;
     double HAvg = (coef1 * HL + coef2 * HR) * divisor;
     double q_2Avg;
     if constexpr (D == 2) q_2Avg = (vAvg[0] * vAvg[0] + vAvg[1] * vAvg[1]) / 2;
     else q_2Avg = (vAvg[0] * vAvg[0] + vAvg[1] * vAvg[1] + vAvg[2] * vAvg[2]) / 2;
-    double cAvg = sqrt((kGamma - 1) * (HAvg - q_2Avg));
+    double cAvg = o.sqrt((kGamma - 1) * (HAvg - q_2Avg));
     double VnAvg = vAvg[AX];
     double lambda[3] = {fabs(VnAvg - cAvg), fabs(VnAvg), fabs(VnAvg + cAvg)};
     double eps = 0.05 * (fabs(VnAvg) + cAvg);
     if (lambda[0] < eps || lambda[1] < eps || lambda[2] < eps) {
-        const Lam3 fx = entropy_fix3(lambda[0], lambda[1], lambda[2], eps);
-        lambda[0] = fx.a;
-        lambda[1] = fx.b;
-        lambda[2] = fx.c;
+        if constexpr (O::spec) {
+            const double e2 = 2.0 * eps, y = o.rcp(e2);
+            for (int i = 0; i < 3; i++) {
+                const double f = o.div_y(lambda[i] * lambda[i] + eps * eps, e2, y);
+                lambda[i] = (lambda[i] < eps) ? f : lambda[i];
+            }
+        } else {
+            const Lam3 fx = entropy_fix3(lambda[0], lambda[1], lambda[2], eps);
+            lambda[0] = fx.a;
+            lambda[1] = fx.b;
+            lambda[2] = fx.c;
+        }
     }
 
     double deltaP = pr - pl, deltaVn = VnR - VnL, deltaRho = rr - rl;
@@ -1630,13 +1908,9 @@ CFD_HD void roe_md(const double *L, const double *R, double *res)
     double Fd[NV];
     // the three quotients by c^2 and 2 c^2 from one correctly rounded
     // reciprocal: (2 c) c = 2 RN(c c) exactly, so x / (2 c c) = RN(x / (c c)) / 2
-    const double cc2 = cAvg * cAvg, icc2 = rcp_rn(cc2);
-    double qc[3];
-    {
-        const double a[3] = {deltaP - rhoAvg * cAvg * deltaVn, deltaP + rhoAvg * cAvg * deltaVn, deltaP},
-                     bb[3] = {cc2, cc2, cc2}, yy[3] = {icc2, icc2, icc2};
-        divs_rn<3>(a, bb, yy, qc);
-    }
+    const double cc2 = cAvg * cAvg, icc2 = o.rcp(cc2);
+    const double qc[3] = {o.div_y(deltaP - rhoAvg * cAvg * deltaVn, cc2, icc2),
+                          o.div_y(deltaP + rhoAvg * cAvg * deltaVn, cc2, icc2), o.div_y(deltaP, cc2, icc2)};
     double c1 = qc[0] / 2;
     Fd[0] = lambda[0] * (c1 * 1);
     for (int i = 0; i < D; i++) Fd[1 + i] = lambda[0] * (c1 * (vAvg[i] - cAvg * n[i]));
@@ -1666,14 +1940,20 @@ CFD_HD void roe_md(const double *L, const double *R, double *res)
 #endif
 }
 
+template <int NV, int AX, int FLUX, class O>
+CFD_HD void riemann(const double *L, const double *R, double *res, O &o, const double *ir)
+{
+    if constexpr (NV == 3) {
+        if constexpr (FLUX == FLUX_HLLC) hllc_1d(L, R, res, o, ir); else roe_1d(L, R, res, o, ir);
+    } else {
+        if constexpr (FLUX == FLUX_HLLC) hllc_md<NV, AX>(L, R, res, o, ir); else roe_md<NV, AX>(L, R, res, o, ir);
+    }
+}
 template <int NV, int AX, int FLUX>
 CFD_HD void riemann(const double *L, const double *R, double *res)
 {
-    if constexpr (NV == 3) {
-        if constexpr (FLUX == FLUX_HLLC) hllc_1d(L, R, res); else roe_1d(L, R, res);
-    } else {
-        if constexpr (FLUX == FLUX_HLLC) hllc_md<NV, AX>(L, R, res); else roe_md<NV, AX>(L, R, res);
-    }
+    OpsIeee o;
+    riemann<NV, AX, FLUX>(L, R, res, o, nullptr);
 }
 
 // Physical (node) flux: fluxSolveEuler1D / fluxSolveEuler2D

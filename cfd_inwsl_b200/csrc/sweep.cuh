@@ -118,6 +118,118 @@ __device__ __noinline__ PrimVals<NV> ghost_prim_ool(const SweepParams &p, const 
     return r;
 }
 
+// What the FP64 sweeps keep of a cell: prim, the cons the reference re-derives
+// from it (primToChar's prologue) and its Roe weights.
+template <int NV>
+struct CellVals {
+    double pr[NV], cs[NV], kw[NV];
+};
+
+template <int NV, int AX, bool RW, class O>
+__device__ __forceinline__ void cell_from_cons(const double *u, CellVals<NV> &c, O &o)
+{
+    const double ir = cons_to_prim<NV>(u, c.pr, o);
+    prim_to_cons<NV>(c.pr, c.cs, o);
+    if constexpr (RW && NV >= 4) EigenBase<NV, AX>::roe_weights(c.pr, c.kw, ir, o);
+}
+
+// Out of line with IEEE operations: operands outside OpsSpec's range, and
+// boundary ghosts (a few cells per line end).
+template <int NV, int AX, bool RW>
+__device__ __noinline__ CellVals<NV> cell_ieee(PrimVals<NV> u)
+{
+    CellVals<NV> c;
+    OpsIeee o;
+    cell_from_cons<NV, AX, RW>(u.v, c, o);
+    return c;
+}
+
+template <int NV, int AX, int NG, bool RW>
+__device__ __noinline__ CellVals<NV> ghost_cell(const SweepParams &p, const BcLine &bl, int k, double tstage)
+{
+    CellVals<NV> c;
+    ghost_prim<NV, NG>(p, bl, k, tstage, c.pr);
+    prim_to_cons<NV>(c.pr, c.cs);
+    if constexpr (RW && NV >= 4) EigenBase<NV, AX>::roe_weights(c.pr, c.kw);
+    return c;
+}
+
+// max wave speed terms of a new state, out of line (IEEE operations): u_d + c
+// over h_d and the two values of the sign test
+template <int NV>
+__device__ __noinline__ PrimVals<5> wave_terms_ieee(PrimVals<NV> u, double h0, double h1, double h2)
+{
+    PrimVals<5> r;
+    double pr[NV];
+    const double hd[3] = {h0, h1, h2};
+    cons_to_prim<NV>(u.v, pr);
+    const double cs = sqrt(kGamma * pr[NV - 1] / pr[0]);
+    for (int d = 0; d < 3; d++) r.v[d] = (d < NV - 2) ? (cs + fabs(pr[1 + d])) / hd[d] : 0.0;
+    r.v[3] = pr[0];
+    r.v[4] = pr[NV - 1];
+    return r;
+}
+
+// The flux of one FP64 face from its stencil in shared memory (sp, sc, kw:
+// the line's prim, cons and Roe weights, PITCH doubles per variable, cell m of
+// the stencil at ring position (s0 + m) & MASK).
+template <int NV, int AX, int FAM, int FLUX, int PITCH, int MASK, bool RW, class O>
+__device__ __forceinline__ void face_flux(const double *sp, const double *sc, const double *kw, int s0, double icst,
+                                          double kap, int posl, double *fx, O &o)
+{
+    int slot[6];
+#pragma unroll
+    for (int m = 0; m < 6; m++) slot[m] = (s0 + m) & MASK;
+    double fl[NV], fr[NV], ir[2] = {0.0, 0.0};
+    if constexpr (NV == 3) {
+        double pr6[6][NV], cs6[6][NV];
+#pragma unroll
+        for (int m = 0; m < 6; m++) {
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                pr6[m][v] = sp[v * PITCH + slot[m]];
+                cs6[m][v] = sc[v * PITCH + slot[m]];
+            }
+        }
+        reconstruct_face<NV, AX, FAM>(pr6, cs6, icst, kap, fl, fr, o, ir);
+    } else {
+        auto csacc = [&](int m, int v) { return sc[v * PITCH + slot[m]]; };
+        auto pracc = [&](int m, int v) { return sp[v * PITCH + slot[m]]; };
+        double kl[NV], kr[NV];
+        if constexpr (RW) {
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                kl[v] = kw[v * PITCH + slot[2]];
+                kr[v] = kw[v * PITCH + slot[3]];
+            }
+        } else {
+            double pl[NV], pr[NV];
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                pl[v] = pracc(2, v);
+                pr[v] = pracc(3, v);
+            }
+            EigenBase<NV, AX>::roe_weights(pl, kl, o.rcp(pl[0]), o);
+            EigenBase<NV, AX>::roe_weights(pr, kr, o.rcp(pr[0]), o);
+        }
+        const EigenBase<NV, AX> eb(kl, kr, o);
+        reconstruct_face_stream<NV, AX, FAM>(eb, csacc, pracc, icst, kap, fl, fr, posl, o, ir);
+    }
+    riemann<NV, AX, FLUX>(fl, fr, fx, o, ir);
+}
+
+// The same out of line with IEEE operations, the positivity fallback and
+// limiters: faces whose operands or states OpsSpec's version does not cover.
+template <int NV, int AX, int FAM, int FLUX, int PITCH, int MASK, bool RW>
+__device__ __noinline__ PrimVals<NV> face_flux_ieee(const double *sp, const double *sc, const double *kw, int s0,
+                                                    double icst, double kap, int posl)
+{
+    PrimVals<NV> r;
+    OpsIeee o;
+    face_flux<NV, AX, FAM, FLUX, PITCH, MASK, RW>(sp, sc, kw, s0, icst, kap, posl, r.v, o);
+    return r;
+}
+
 #ifndef CFD_SWEEP_MINB
 #define CFD_SWEEP_MINB 2
 #endif
@@ -278,6 +390,35 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
         bool ok; long long base; int lid;
         if (PREC == 1 && l == tl) own_line(ok, base, lid);
         else line_of(l, ok, base, lid);
+        int slot = ring(P - s_begin + HG);
+        if constexpr (PREC == 0) {
+            CellVals<NV> c;
+            if (!ok) {  // past the last line: any admissible state, never read back
+#pragma unroll
+                for (int v = 0; v < NV; v++) c.pr[v] = c.cs[v] = c.kw[v] = (v == 0 || v == NV - 1) ? 1.0 : 0.0;
+                c.cs[NV - 1] = 2.5;
+                c.kw[NV - 1] = 3.5;
+            } else if (P >= 0 && P < nd) {
+                PrimVals<NV> u;
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    u.v[v] = staged ? stg[v * NT + threadIdx.x] : __ldg(p.u + v * p.ncell + base + (long long)P * sAX);
+                OpsSpec o;
+                cell_from_cons<NV, AX, SH::RW>(u.v, c, o);
+                if (!o.ok) c = cell_ieee<NV, AX, SH::RW>(u);
+            } else {
+                const bool lo = P < 0;
+                const int k = lo ? -P - 1 : P - nd;
+                c = ghost_cell<NV, AX, HG, SH::RW>(p, lo ? p.bc_lo[lid] : p.bc_hi[lid], k > HG - 1 ? HG - 1 : k, tstage);
+            }
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                sp[(v * W + l) * LSP + slot] = c.pr[v];
+                sc[(v * W + l) * LSP + slot] = c.cs[v];
+                if constexpr (SH::RW) skw[(v * W + l) * LSP + slot] = c.kw[v];
+            }
+            return;
+        }
         double pr[NV];
         double cs[NV];
         bool have_cs = false;  // the mixed form takes interior cells' cons as loaded
@@ -307,13 +448,6 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
             for (int v = 0; v < NV; v++) pr[v] = g.v[v];
         }
         if (!have_cs) prim_to_cons<NV>(pr, cs);  // as the reference's primToChar re-derives them
-        int slot = ring(P - s_begin + HG);
-        if constexpr (SH::RW) {
-            double kw[NV];
-            EigenBase<NV, AX>::roe_weights(pr, kw);
-#pragma unroll
-            for (int v = 0; v < NV; v++) skw[(v * W + l) * LSP + slot] = kw[v];
-        }
 #pragma unroll
         for (int v = 0; v < NV; v++) {
             sp[(v * W + l) * LSP + slot] = pr[v];
@@ -327,57 +461,43 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
 
     // Face j lies between cells j-1 and j (x_{j-1/2}); stencil cells j-3..j+2.
     auto face = [&](int l, int j) {
-        int slot[6];
+        double fx[NV];
+        const double *spl = sp + l * LSP, *scl = sc + l * LSP;
+        if constexpr (PREC == 0) {
+            const int s0 = j - 3 - s_begin + HG;
+            OpsSpec o;
+            face_flux<NV, AX, FAM, FLUX, W * LSP, R - 1, SH::RW>(spl, scl, skw + l * LSP, s0, p.icst, p.icst_k, p.posl, fx,
+                                                                 o);
+            if (!o.ok) {
+                const PrimVals<NV> r = face_flux_ieee<NV, AX, FAM, FLUX, W * LSP, R - 1, SH::RW>(
+                    spl, scl, skw + l * LSP, s0, p.icst, p.icst_k, p.posl);
 #pragma unroll
-        for (int m = 0; m < 6; m++) slot[m] = ring(j - 3 + m - s_begin + HG);
-        double fl[NV], fr[NV], fx[NV];
-        if constexpr (NV == 3) {
-            double pr6[6][NV], cs6[6][NV];
-#pragma unroll
-            for (int m = 0; m < 6; m++) {
-#pragma unroll
-                for (int v = 0; v < NV; v++) {
-                    pr6[m][v] = sp[(v * W + l) * LSP + slot[m]];
-                    cs6[m][v] = sc[(v * W + l) * LSP + slot[m]];
-                }
+                for (int v = 0; v < NV; v++) fx[v] = r.v[v];
             }
-            reconstruct_face<NV, AX, FAM>(pr6, cs6, p.icst, p.icst_k, fl, fr);
         } else {
-            const double *spl = sp + l * LSP, *scl = sc + l * LSP;
+            int slot[6];
+#pragma unroll
+            for (int m = 0; m < 6; m++) slot[m] = ring(j - 3 + m - s_begin + HG);
+            double fl[NV], fr[NV];
             auto csacc = [&](int m, int v) { return scl[v * W * LSP + slot[m]]; };
             auto pracc = [&](int m, int v) { return spl[v * W * LSP + slot[m]]; };
-            if constexpr (PREC == 1 && FAM != FAM_RESEARCH) {
-                const float2 *hll = shl + l * LSP;
-                // the FP32 hi/lo split of each stencil cell's cons
-                auto hlacc = [&](int m, int v) {
-                    return hll[v * W * LSP + slot[m]];
+            const float2 *hll = shl + l * LSP;
+            // the FP32 hi/lo split of each stencil cell's cons
+            auto hlacc = [&](int m, int v) {
+                return hll[v * W * LSP + slot[m]];
+            };
+            if constexpr (SH::HL_CS) {
+                auto hlcs = [&](int m, int v) {
+                    const float2 t = hlacc(m, v);
+                    return (double)t.x + (double)t.y;
                 };
-                if constexpr (SH::HL_CS) {
-                    auto hlcs = [&](int m, int v) {
-                        const float2 t = hlacc(m, v);
-                        return (double)t.x + (double)t.y;
-                    };
-                    reconstruct_face_mixed<NV, AX, FAM>(hlcs, pracc, hlacc, p.icst, p.icst_k, fl, fr);
-                } else {
-                    reconstruct_face_mixed<NV, AX, FAM>(csacc, pracc, hlacc, p.icst, p.icst_k, fl, fr);
-                }
-            } else if constexpr (SH::RW) {
-                const double *kwl = skw + l * LSP;
-                double kl[NV], kr[NV];
-#pragma unroll
-                for (int v = 0; v < NV; v++) {
-                    kl[v] = kwl[v * W * LSP + slot[2]];
-                    kr[v] = kwl[v * W * LSP + slot[3]];
-                }
-                const EigenBase<NV, AX> eb(kl, kr);
-                reconstruct_face_stream<NV, AX, FAM>(eb, csacc, pracc, p.icst, p.icst_k, fl, fr, p.posl);
+                reconstruct_face_mixed<NV, AX, FAM>(hlcs, pracc, hlacc, p.icst, p.icst_k, fl, fr);
             } else {
-                reconstruct_face_stream<NV, AX, FAM>(csacc, pracc, p.icst, p.icst_k, fl, fr, p.posl);
+                reconstruct_face_mixed<NV, AX, FAM>(csacc, pracc, hlacc, p.icst, p.icst_k, fl, fr);
             }
+            if constexpr (FLUX == FLUX_ROE) roe_md_mixed<NV, AX>(fl, fr, fx);
+            else hllc_md_mixed<NV, AX>(fl, fr, fx);
         }
-        if constexpr (PREC == 1 && FLUX == FLUX_ROE && NV >= 4) roe_md_mixed<NV, AX>(fl, fr, fx);
-        else if constexpr (PREC == 1 && FLUX == FLUX_HLLC && NV >= 4) hllc_md_mixed<NV, AX>(fl, fr, fx);
-        else riemann<NV, AX, FLUX>(fl, fr, fx);
         int fslot = fring(j - s_begin + FO);
 #pragma unroll
         for (int v = 0; v < NV; v++) sf[(v * W + l) * LSF + fslot] = fx[v];
@@ -487,15 +607,23 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
                     dd[v] = mnd6(fnm[v], fnp[v], fv[fs[0]], fv[fs[1]], fv[fs[2]], fv[fs[3]], p.h, inv_h);
                 }
 #else
-                double num[NV], hh[NV], ihh[NV];
+                DivN<NV> num;
+                OpsSpec o;
+                o.need(OpsSpec::in_range(p.h));
 #pragma unroll
                 for (int v = 0; v < NV; v++) {
                     const double *fv = sf + (v * W + tl) * LSF;
-                    num[v] = mnd6_num(fnm[v], fnp[v], fv[fs[0]], fv[fs[1]], fv[fs[2]], fv[fs[3]]);
-                    hh[v] = p.h;
-                    ihh[v] = inv_h;
+                    num.v[v] = mnd6_num(fnm[v], fnp[v], fv[fs[0]], fv[fs[1]], fv[fs[2]], fv[fs[3]]);
+                    dd[v] = o.div_y(num.v[v], p.h, inv_h);
                 }
-                divs_rn<NV>(num, hh, ihh, dd);
+                if (!o.ok) {
+                    DivN<NV> hh;
+#pragma unroll
+                    for (int v = 0; v < NV; v++) hh.v[v] = p.h;
+                    const DivN<NV> q = divs_ieee<NV>(num, hh);
+#pragma unroll
+                    for (int v = 0; v < NV; v++) dd[v] = q.v[v];
+                }
 #endif
             }
             double uo[NV];
@@ -538,7 +666,38 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
 #pragma unroll
                 for (int v = 0; v < NV; v++) fin = fin && isfinite(uo[v]);
                 if (!fin) err |= ERR_NONFINITE;
-                if (p.want_reduce) {
+                if constexpr (PREC == 0) {
+                    if (p.want_reduce) {
+                        double pr[NV], lam[3] = {0.0, 0.0, 0.0};
+                        OpsSpec o;
+                        const double ir = cons_to_prim<NV>(uo, pr, o);
+                        (void)ir;
+#if defined(CFD_FAST)
+                        const double cs = o.sqrt(o.div(kGamma * pr[NV - 1], pr[0]));
+#else
+                        const double cs = o.sqrt(o.div_y(kGamma * pr[NV - 1], pr[0], ir));
+#endif
+#pragma unroll
+                        for (int d = 0; d < NV - 2; d++) {
+                            const double a = cs + fabs(pr[1 + d]);
+                            o.need(OpsSpec::in_range(a) & OpsSpec::in_range(p.hdir[d]));
+                            lam[d] = OpsSpec::quot(a, p.hdir[d], inv_hdir[d]);
+                        }
+                        if (!o.ok) {
+                            PrimVals<NV> u;
+#pragma unroll
+                            for (int v = 0; v < NV; v++) u.v[v] = uo[v];
+                            const PrimVals<5> w = wave_terms_ieee<NV>(u, p.hdir[0], p.hdir[1], p.hdir[2]);
+#pragma unroll
+                            for (int d = 0; d < NV - 2; d++) lam[d] = w.v[d];
+                            pr[0] = w.v[3];
+                            pr[NV - 1] = w.v[4];
+                        }
+                        if (!(pr[0] > 0.0) || !(pr[NV - 1] > 0.0)) err |= ERR_NEGATIVE;
+#pragma unroll
+                        for (int d = 0; d < NV - 2; d++) red_lam[d] = fmax(red_lam[d], lam[d]);
+                    }
+                } else if (p.want_reduce) {
                     double pr[NV];
                     cons_to_prim<NV>(uo, pr);
                     if (!(pr[0] > 0.0) || !(pr[NV - 1] > 0.0)) err |= ERR_NEGATIVE;
