@@ -7,6 +7,12 @@
 // FMAs and, where CFD_FAST is defined, a few algebraic rewrites that trade the
 // last ulp for fewer divisions; those are marked "fast path".
 //
+// Products with the zeros and ones of a unit normal are not formed: x + 0 y and
+// 1 x round to x for finite y, and the sign of a zero sum cannot reach the
+// result, because the first direction's difference enters the right-hand side
+// as 0.0 + d, which is never -0. nvcc has to keep such operations; they were
+// about a tenth of a face's FP64 instructions.
+//
 // Layout conventions: prim = (rho, u, v[, w], p), cons = (rho, rho u, rho v
 // [, rho w], rho E); NV = 3 (1D), 4 (2D), 5 (3D). AX is the sweep axis
 // (0 = x, 1 = y, 2 = z); the face normal is the unit vector along AX.
@@ -387,11 +393,27 @@ CFD_HD double teno_select(unsigned flag, double q0, double q1, double q2, double
 // the early answer is the reference's own flag 0, bit for bit.
 inline double teno_kappa(double c) { return c > 0.0 ? ::pow(3.3 * c, 1.0 / 6.0) : 0.0; }
 
+//
+// The sums use s_k = beta_k: with 0 <= s_min <= s_max the ratio only grows when
+// eps is added to both (its logarithm's derivative is g(s_min) - g(s_max) >= 0,
+// g(x) = 1/x - 1/(x + tau)), and where a product underflows tau < 1e-153, so
+// that every measure is 1 beside eps = 1e-40. The measures are sums of squares:
+// their order is that of their bits, compared as integers off the FP64 pipe
+// (a NaN ends up in one of the products and fails the test).
 CFD_HD bool teno_z_all_kept(double s0, double s1, double s2, double tau, double kap)
 {
+#if defined(__CUDA_ARCH__)
+    const long long i0 = __double_as_longlong(s0), i1 = __double_as_longlong(s1), i2 = __double_as_longlong(s2);
+    const long long ia = i0 < i1 ? i0 : i1, ib = i0 < i1 ? i1 : i0;
+    const double smin = __longlong_as_double(ia < i2 ? ia : i2), smax = __longlong_as_double(ib < i2 ? i2 : ib);
+    const double lhs = (smax + tau) * smin, rhs = (smin + tau) * smax;
+    // rhs < 2^996 (about 1e300), on the exponent bits
+    return (__double2hiint(rhs) < (int)(2019u << 20)) & (lhs >= kap * rhs);
+#else
     const double smin = fmin(s0, fmin(s1, s2)), smax = fmax(s0, fmax(s1, s2));
     const double lhs = (smax + tau) * smin, rhs = (smin + tau) * smax;
     return rhs < 1e300 && lhs >= kap * rhs;
+#endif
 }
 
 // Interpolator families. Each selector entry of the reference maps onto one
@@ -719,9 +741,7 @@ CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, doub
         s = eps + b0; b0 = o.rcp(s * s) * (1.0 / 16.0);
         s = eps + b1; b1 = o.div_pos(5.0 / 8.0, s * s);
         s = eps + b2; b2 = o.div_pos(5.0 / 16.0, s * s);
-        double sumbeta = b0, result = 0.0;  // 0 + b0 = b0 (b0 > 0)
-        sumbeta += b1; sumbeta += b2;
-        result += b0 * u0; result += b1 * u1; result += b2 * u2;
+        const double sumbeta = b0 + b1 + b2, result = b0 * u0 + b1 * u1 + b2 * u2;
         return o.div(result, sumbeta);
 #endif
     } else if constexpr (FAM == FAM_WENOZ) {
@@ -734,19 +754,15 @@ CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, doub
         x = o.div(tau, b0 + eps); b0 = (1.0 / 16.0) * (1.0 + x * x);
         x = o.div(tau, b1 + eps); b1 = (5.0 / 8.0) * (1.0 + x * x);
         x = o.div(tau, b2 + eps); b2 = (5.0 / 16.0) * (1.0 + x * x);
-        double sumbeta = b0, result = 0.0;  // 0 + b0 = b0 (b0 > 0)
-        sumbeta += b1; sumbeta += b2;
-        result += b0 * u0; result += b1 * u1; result += b2 * u2;
+        const double sumbeta = b0 + b1 + b2, result = b0 * u0 + b1 * u1 + b2 * u2;
         return o.div(result, sumbeta);
     } else if constexpr (FAM == FAM_TENOZ) {
         // TENO5 with the Z-type measure (1 + tau/(beta_k + eps))^6 and the
         // cutoff measure_k < c * sum_j measure_j (Teno5_Z: interScheme.hpp:384-452).
-        const double eps = 1e-40;
         double b0, b1, b2;
         smoothness3(q0, q1, q2, q3, q4, b0, b1, b2);
-        double tau = fabs(b2 - b0), t;
-        (void)t;
-        if (kap > 0.0 && teno_z_all_kept(b0 + eps, b1 + eps, b2 + eps, tau, kap))
+        double tau = fabs(b2 - b0);
+        if (kap > 0.0 && teno_z_all_kept(b0, b1, b2, tau, kap))
             return teno_select(0u, q0, q1, q2, q3, q4);
         return teno_select(teno_z_flag(b0, b1, b2, tau, c), q0, q1, q2, q3, q4);
     } else if constexpr (FAM == FAM_TENOCONG) {
@@ -1343,13 +1359,9 @@ struct EigenBase {
         v = (kl[2] + kr[2]) * divisor;
         w = (D == 3) ? (kl[3] + kr[3]) * divisor : 0.0;
         const double ht = (kl[NV - 1] + kr[NV - 1]) * divisor;
-        if constexpr (D == 2) {
-            Vn = nx * u + ny * v;
-            ek = (u * u + v * v) / 2;
-        } else {
-            Vn = nx * u + ny * v + nz * w;
-            ek = (u * u + v * v + w * w) / 2;
-        }
+        Vn = (AX == 0) ? u : (AX == 1) ? v : w;
+        if constexpr (D == 2) ek = (u * u + v * v) / 2;
+        else ek = (u * u + v * v + w * w) / 2;
         h = ht - ek;
 #if defined(CFD_FAST)
         // 1/c = rsqrt(c^2), 1/h = (gamma - 1) / c^2
@@ -1374,16 +1386,18 @@ struct EigenBase {
     CFD_HD double dc(double a) const { return a * ic; }
     CFD_HD double dh(double a) const { return a * ih; }
 #endif
-    // (s n_i) / c for a unit normal component n_i (0 or 1) and s = -1 or 1:
-    // the correctly rounded 1/c with the sign, or a signed zero, exactly as
-    // the division rounds it
-    CFD_HD double sn_c(double s, double n) const { return (s * n) * ic; }
+    // ((s n_i) / c - x) / 2 for a unit normal component n_i (0 or 1), s = -1 or 1
+    // and x = (velocity component) / h
+    CFD_HD double half_sn_c(double s, double n, double x) const
+    {
+        return (n == 0.0) ? -0.5 * x : (s < 0.0) ? (-ic - x) / 2 : (ic - x) / 2;
+    }
     // left eigenvector k, column m (eigenSystem.cpp:53-68 and the 3D extension)
     CFD_HD double L(int k, int m) const
     {
         constexpr int E = NV - 1;
         if (k == 0) {
-            if (AX != 2) return m == 0 ? (-ny * u + nx * v) : m == 1 ? ny : m == 2 ? (-nx) : (m == E ? 0 : 0.0);
+            if (AX != 2) return m == 0 ? (AX == 0 ? v : -u) : m == 1 ? ny : m == 2 ? (-nx) : (m == E ? 0 : 0.0);
             return m == 0 ? -u : m == 1 ? 1.0 : 0.0;
         }
         if (k == 1) return m == 0 ? (h - ek) : m == 1 ? u : m == 2 ? v : m == E ? -1.0 : w;
@@ -1393,15 +1407,15 @@ struct EigenBase {
             if (m == E) return 0.5 * ih;
 #if defined(CFD_FAST)
             if (m == 0) return (k == 2) ? (dc(Vn) + dh(ek)) / 2 : (dc(-Vn) + dh(ek)) / 2;
-            if (m == 1) return (dc(s * nx) - dh(u)) / 2;
-            if (m == 2) return (dc(s * ny) - dh(v)) / 2;
-            return (dc(s * nz) - dh(w)) / 2;
+            if (m == 1) return half_sn_c(s, nx, dh(u));
+            if (m == 2) return half_sn_c(s, ny, dh(v));
+            return half_sn_c(s, nz, dh(w));
 #else
             // (-Vn) / c = -(Vn / c) exactly
             if (m == 0) return (k == 2) ? (Vc + ekh) / 2 : (-Vc + ekh) / 2;
-            if (m == 1) return (sn_c(s, nx) - uh) / 2;
-            if (m == 2) return (sn_c(s, ny) - vh) / 2;
-            return (sn_c(s, nz) - wh) / 2;
+            if (m == 1) return half_sn_c(s, nx, uh);
+            if (m == 2) return half_sn_c(s, ny, vh);
+            return half_sn_c(s, nz, wh);
 #endif
         }
         // k == 4: second shear wave (3D only)
@@ -1413,7 +1427,7 @@ struct EigenBase {
     {
         constexpr int E = NV - 1;
         if (k == 0) {
-            if (AX != 2) return i == 0 ? 0.0 : i == 1 ? ny : i == 2 ? -nx : i == E ? ny * u - nx * v : 0.0;
+            if (AX != 2) return i == 0 ? 0.0 : i == 1 ? ny : i == 2 ? -nx : i == E ? (AX == 0 ? -v : u) : 0.0;
             return i == 1 ? 1.0 : i == E ? u : 0.0;
         }
 #if defined(CFD_FAST)
@@ -1425,10 +1439,10 @@ struct EigenBase {
             const double s = (k == 2) ? -1.0 : 1.0;
             if (i == 0) return 1.0;
             if (i == E) return (k == 2) ? h + ek - Vn * c : h + ek + Vn * c;
-            if (i == 1) return (k == 2) ? u - nx * c : u + nx * c;
-            if (i == 2) return (k == 2) ? v - ny * c : v + ny * c;
             (void)s;
-            return (k == 2) ? w - nz * c : w + nz * c;
+            if (i == 1) return (AX != 0) ? u : (k == 2) ? u - c : u + c;
+            if (i == 2) return (AX != 1) ? v : (k == 2) ? v - c : v + c;
+            return (AX != 2) ? w : (k == 2) ? w - c : w + c;
         }
         if (AX != 2) return i == 3 ? 1.0 : i == 4 ? w : 0.0;
         return i == 2 ? 1.0 : i == 4 ? v : 0.0;
@@ -1462,6 +1476,13 @@ CFD_HD void reconstruct_face_stream(const EigenBase<NV, AX> &eb, const CS &cs, c
 #pragma unroll
         for (int j = 0; j < 6; j++) {
             // primToChar's order: rut L1 + rvt L2 [+ rwt L3] + ret LE + rt L0
+            if (k == 0 || k == 4) {
+                // shear waves: one momentum component (sign t) and rho l0
+                constexpr int M0 = (AX == 0) ? 2 : 1, M4 = (AX == 2) ? 2 : (NV == 5 ? 3 : 0);
+                const double mt = cs(j, k == 0 ? M0 : M4);
+                q[j] = ((k == 0 && AX == 0) ? -mt : mt) + cs(j, 0) * l[0];
+                continue;
+            }
             double a = cs(j, 1) * l[1] + cs(j, 2) * l[2];
 #pragma unroll
             for (int m = 3; m < NV; m++) a = a + cs(j, m) * l[m];
@@ -1484,6 +1505,9 @@ CFD_HD void reconstruct_face_stream(const EigenBase<NV, AX> &eb, const CS &cs, c
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             const double r = eb.R(i, k);
+            // the shear waves carry one momentum component and its energy
+            if (k == 0 && i != ((AX == 0) ? 2 : 1) && i != NV - 1) continue;
+            if (k == 4 && i != ((AX == 2) ? 2 : 3) && i != NV - 1) continue;
             if (kk == 0) {
                 cl[i] = QL * r;
                 cr[i] = QR * r;
@@ -1659,7 +1683,6 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const d
 {
     constexpr int D = NV - 2, E = NV - 1;
     const double gamma = kGamma;
-    const double n[3] = {AX == 0 ? 1.0 : 0.0, AX == 1 ? 1.0 : 0.0, AX == 2 ? 1.0 : 0.0};
     double rl = L[0], rr = R[0], pl = L[E], pr = R[E];
     const double *vl = L + 1, *vr = R + 1;
     double HL, HR;
@@ -1719,13 +1742,13 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const d
         for (int i = 0; i < D; i++) U[1 + i] = r * v[i];
         U[E] = r * H - p;
         F[0] = r * Vn;
-        for (int i = 0; i < D; i++) F[1 + i] = r * v[i] * Vn + p * n[i];
+        for (int i = 0; i < D; i++) F[1 + i] = (i == AX) ? r * v[i] * Vn + p : r * v[i] * Vn;
         F[E] = r * H * Vn;
         const double SV = neg ? -(S - Vn) : S - Vn, SS = neg ? -(S - Sstar) : S - Sstar;
         double Usf = O::spec ? o.div(SV, SS) : (S - Vn) / (S - Sstar);
         const double pS = O::spec ? o.div(neg ? -p : p, SV) : p / (S - Vn);
         Ustar[0] = Usf * r;
-        for (int i = 0; i < D; i++) Ustar[1 + i] = Usf * (Sstar * n[i] + v[i] * (1.0 - n[i])) * r;
+        for (int i = 0; i < D; i++) Ustar[1 + i] = Usf * ((i == AX) ? Sstar : v[i]) * r;
         Ustar[E] = Usf * (U[E] + (Sstar - Vn) * (r * Sstar + pS));
         for (int i = 0; i < NV; i++) {
             double f = F[i] + S * (Ustar[i] - U[i]);
@@ -1735,7 +1758,7 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const d
     };
     if (SL > 0) {
         res[0] = rl * VnL;
-        for (int i = 0; i < D; i++) res[1 + i] = rl * vl[i] * VnL + pl * n[i];
+        for (int i = 0; i < D; i++) res[1 + i] = (i == AX) ? rl * vl[i] * VnL + pl : rl * vl[i] * VnL;
         res[E] = rl * HL * VnL;
     } else if (Sstar > 0 || Sstar == 0 || SR > 0) {
         // The star-region branches of the reference in one body: S* > 0 takes
@@ -1755,7 +1778,7 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const d
         }
     } else {
         res[0] = rr * VnR;
-        for (int i = 0; i < D; i++) res[1 + i] = rr * vr[i] * VnR + pr * n[i];
+        for (int i = 0; i < D; i++) res[1 + i] = (i == AX) ? rr * vr[i] * VnR + pr : rr * vr[i] * VnR;
         res[E] = rr * HR * VnR;
     }
 }
@@ -1769,7 +1792,6 @@ template <int NV, int AX, class O>
 CFD_HD void roe_md_fast(const double *L, const double *R, double *res, O &o)
 {
     constexpr int D = NV - 2, E = NV - 1;
-    const double n[3] = {AX == 0 ? 1.0 : 0.0, AX == 1 ? 1.0 : 0.0, AX == 2 ? 1.0 : 0.0};
     const double rl = L[0], rr = R[0], pl = L[E], pr = R[E];
     const double *vl = L + 1, *vr = R + 1;
     double kl = vl[0] * vl[0] + vl[1] * vl[1], kr = vr[0] * vr[0] + vr[1] * vr[1];
@@ -1777,7 +1799,8 @@ CFD_HD void roe_md_fast(const double *L, const double *R, double *res, O &o)
     const double VnL = vl[AX], VnR = vr[AX];
     double Fc[NV];
     Fc[0] = rl * VnL + rr * VnR;
-    for (int i = 0; i < D; i++) Fc[1 + i] = rl * vl[i] * VnL + rr * vr[i] * VnR + (pl + pr) * n[i];
+    for (int i = 0; i < D; i++) Fc[1 + i] = rl * vl[i] * VnL + rr * vr[i] * VnR;
+    Fc[1 + AX] += pl + pr;
     Fc[E] = (0.5 * rl * kl + kG1 * pl) * VnL + (0.5 * rr * kr + kG1 * pr) * VnR;
 
     const double ir1 = o.rsqrt(rl), ir2 = o.rsqrt(rr);
@@ -1811,9 +1834,13 @@ CFD_HD void roe_md_fast(const double *L, const double *R, double *res, O &o)
     Fd[0] = a1 + a3 + a2;
     double tE = 0.0;
     for (int i = 0; i < D; i++) {
-        const double ti = (i == AX) ? 0.0 : vr[i] - vl[i];
-        Fd[1 + i] = a1 * (vAvg[i] - cAvg * n[i]) + a3 * (vAvg[i] + cAvg * n[i]) + a2 * vAvg[i] + l1r * ti;
-        if (i != AX) tE += vAvg[i] * ti;
+        if (i == AX) {
+            Fd[1 + i] = a1 * (vAvg[i] - cAvg) + a3 * (vAvg[i] + cAvg) + a2 * vAvg[i];
+        } else {
+            const double ti = vr[i] - vl[i];
+            Fd[1 + i] = a1 * vAvg[i] + a3 * vAvg[i] + a2 * vAvg[i] + l1r * ti;
+            tE += vAvg[i] * ti;
+        }
     }
     Fd[E] = a1 * (HAvg - cAvg * VnAvg) + a3 * (HAvg + cAvg * VnAvg) + a2 * q_2Avg + l1r * tE;
     for (int i = 0; i < NV; i++) res[i] = 0.5 * (Fc[i] - Fd[i]);
@@ -1849,7 +1876,6 @@ CFD_HD void roe_md(const double *L, const double *R, double *res, O &o, const do
     roe_md_fast<NV, AX>(L, R, res, o);
 #else
     constexpr int D = NV - 2, E = NV - 1;
-    const double n[3] = {AX == 0 ? 1.0 : 0.0, AX == 1 ? 1.0 : 0.0, AX == 2 ? 1.0 : 0.0};
     double rl = L[0], rr = R[0], pl = L[E], pr = R[E];
     const double *vl = L + 1, *vr = R + 1;
     double HL, HR;
@@ -1868,10 +1894,10 @@ CFD_HD void roe_md(const double *L, const double *R, double *res, O &o, const do
     double VnL = vl[AX], VnR = vr[AX];
     double FcL[NV], FcR[NV];
     FcL[0] = rl * VnL;
-    for (int i = 0; i < D; i++) FcL[1 + i] = rl * vl[i] * VnL + pl * n[i];
+    for (int i = 0; i < D; i++) FcL[1 + i] = (i == AX) ? rl * vl[i] * VnL + pl : rl * vl[i] * VnL;
     FcL[E] = rl * HL * VnL;
     FcR[0] = rr * VnR;
-    for (int i = 0; i < D; i++) FcR[1 + i] = rr * vr[i] * VnR + pr * n[i];
+    for (int i = 0; i < D; i++) FcR[1 + i] = (i == AX) ? rr * vr[i] * VnR + pr : rr * vr[i] * VnR;
     FcR[E] = rr * HR * VnR;
 
     double coef1 = o.sqrt(rl), coef2 = o.sqrt(rr);
@@ -1913,23 +1939,22 @@ CFD_HD void roe_md(const double *L, const double *R, double *res, O &o, const do
                           o.div_y(deltaP + rhoAvg * cAvg * deltaVn, cc2, icc2), o.div_y(deltaP, cc2, icc2)};
     double c1 = qc[0] / 2;
     Fd[0] = lambda[0] * (c1 * 1);
-    for (int i = 0; i < D; i++) Fd[1 + i] = lambda[0] * (c1 * (vAvg[i] - cAvg * n[i]));
+    for (int i = 0; i < D; i++) Fd[1 + i] = lambda[0] * (c1 * ((i == AX) ? vAvg[i] - cAvg : vAvg[i]));
     Fd[E] = lambda[0] * (c1 * (HAvg - cAvg * VnAvg));
 
     double cc = qc[1] / 2;
     Fd[0] += lambda[2] * (cc * 1);
-    for (int i = 0; i < D; i++) Fd[1 + i] += lambda[2] * (cc * (vAvg[i] + cAvg * n[i]));
+    for (int i = 0; i < D; i++) Fd[1 + i] += lambda[2] * (cc * ((i == AX) ? vAvg[i] + cAvg : vAvg[i]));
     Fd[E] += lambda[2] * (cc * (HAvg + cAvg * VnAvg));
 
     double c2 = deltaRho - qc[2];
-    Fd[0] += lambda[1] * (c2 * 1.0 + rhoAvg * 0.0);
+    Fd[0] += lambda[1] * c2;
     // tangential components carry rhoAvg * dv_i, the normal one 0
     // (fluxSchemes.hpp:526-528 for axis normals).
     double tE = 0.0;
     bool first = true;
     for (int i = 0; i < D; i++) {
-        double ti = (i == AX) ? 0 : dv[i];
-        Fd[1 + i] += lambda[1] * (c2 * vAvg[i] + rhoAvg * ti);
+        Fd[1 + i] += lambda[1] * ((i == AX) ? c2 * vAvg[i] : c2 * vAvg[i] + rhoAvg * dv[i]);
         if (i != AX) {
             double term = vAvg[i] * dv[i];
             if (first) { tE = term; first = false; } else tE = tE + term;
@@ -1968,13 +1993,10 @@ CFD_HD void node_flux(const double *p, double *f)
         f[2] = (kGamma / (kGamma - 1) * pp + r * (u * u) / 2) * u;
     } else {
         constexpr int D = NV - 2, E = NV - 1;
-        const double n[3] = {AX == 0 ? 1.0 : 0.0, AX == 1 ? 1.0 : 0.0, AX == 2 ? 1.0 : 0.0};
         double r = p[0], pp = p[E];
-        double Vn;
-        if constexpr (D == 2) Vn = (p[1] * n[0] + p[2] * n[1]);
-        else Vn = (p[1] * n[0] + p[2] * n[1] + p[3] * n[2]);
+        const double Vn = p[1 + AX];
         f[0] = r * Vn;
-        for (int i = 0; i < D; i++) f[1 + i] = r * p[1 + i] * Vn + n[i] * pp;
+        for (int i = 0; i < D; i++) f[1 + i] = (i == AX) ? r * p[1 + i] * Vn + pp : r * p[1 + i] * Vn;
         double q2;
         if constexpr (D == 2) q2 = (p[1] * p[1] + p[2] * p[2]);
         else q2 = (p[1] * p[1] + p[2] * p[2] + p[3] * p[3]);
