@@ -194,6 +194,15 @@ struct OpsIeee {
     CFD_HD double div_pos(double a, double b) { return a / b; }
     CFD_HD double sqrt(double x) { return ::sqrt(x); }
     CFD_HD void need(bool) {}
+    // forms without a range check of their own (see OpsSpec)
+    CFD_HD double rcp_in(double b) { return rcp(b); }
+    CFD_HD double div_y_in(double a, double b, double y) { return div_y(a, b, y); }
+    CFD_HD double sqrt_in(double x) { return ::sqrt(x); }
+    CFD_HD double div_in(double a, double b) { return a / b; }
+    CFD_HD double div_b_in(double a, double b) { return a / b; }
+    CFD_HD void need_pos(double) {}
+    CFD_HD void need_sq(double) {}
+    CFD_HD void need_below(double, double, double) {}
 };
 
 #if defined(__CUDACC__)
@@ -226,6 +235,22 @@ struct OpsSpec {
         e = __fma_ru(e, e, e);
         return fma(y, e, y);
     }
+    // Checks shared by several operations, whose _in forms then make none:
+    // a positive value; a component whose square (summed with others') is
+    // divided too, so 0 or 2^-399 <= |x| < 2^240; three positive values whose
+    // lower bounds are known.
+    __device__ __forceinline__ void need_pos(double x) { need(in_range(x)); }
+    __device__ __forceinline__ void need_sq(double x)
+    {
+        const unsigned t = (unsigned)__double2hiint(x) & 0x7fffffffu, lo = (unsigned)__double2loint(x);
+        need((t - (624u << 20) < (639u << 20)) | ((t | lo) == 0u));
+    }
+    __device__ __forceinline__ void need_below(double a, double b, double c)
+    {
+        const unsigned m = __vimax3_u32((unsigned)__double2hiint(a), (unsigned)__double2hiint(b),
+                                        (unsigned)__double2hiint(c));
+        need(m < (1223u << 20));
+    }
     // RN(a/b) from y = 1/b, b > 0. The residual carries the sign that keeps a
     // quotient of a zero dividend at that zero.
     static __device__ __forceinline__ double quot(double a, double b, double y)
@@ -233,9 +258,8 @@ struct OpsSpec {
         const double q = a * y;
         return fma(-fma(b, q, -a), y, q);
     }
-    __device__ __forceinline__ double rcp(double b)
+    __device__ __forceinline__ double rcp_in(double b)
     {
-        need(in_range(b));
         const double y = rcp_near(b);
 #if defined(CFD_FAST)
         return y;
@@ -243,14 +267,32 @@ struct OpsSpec {
         return fma(fma(-b, y, 1.0), y, y);
 #endif
     }
-    __device__ __forceinline__ double div_y(double a, double b, double y)
+    __device__ __forceinline__ double rcp(double b)
+    {
+        need(in_range(b));
+        return rcp_in(b);
+    }
+    __device__ __forceinline__ double div_y_in(double a, double b, double y)
     {
 #if defined(CFD_FAST)
         return a * y;
 #else
-        need(in_range_or_0(a));
         return quot(a, b, y);
 #endif
+    }
+    __device__ __forceinline__ double div_y(double a, double b, double y)
+    {
+#if !defined(CFD_FAST)
+        need(in_range_or_0(a));
+#endif
+        return div_y_in(a, b, y);
+    }
+    __device__ __forceinline__ double div_in(double a, double b) { return quot(a, b, rcp_near(b)); }
+    // a / b for a b known to be in range
+    __device__ __forceinline__ double div_b_in(double a, double b)
+    {
+        need(in_range_or_0(a));
+        return div_in(a, b);
     }
     // a / b for b > 0 (any other b takes the out-of-line path)
     __device__ __forceinline__ double div(double a, double b)
@@ -274,6 +316,10 @@ struct OpsSpec {
     __device__ __forceinline__ double sqrt(double x)
     {
         need(in_range(x));
+        return sqrt_in(x);
+    }
+    __device__ __forceinline__ double sqrt_in(double x)
+    {
         const double y = rsqrt_seed(x);
         double g = x * y, h = 0.5 * y;
         const double r = fma(-g, h, 0.5);
@@ -397,15 +443,19 @@ inline double teno_kappa(double c) { return c > 0.0 ? ::pow(3.3 * c, 1.0 / 6.0) 
 // The sums use s_k = beta_k: with 0 <= s_min <= s_max the ratio only grows when
 // eps is added to both (its logarithm's derivative is g(s_min) - g(s_max) >= 0,
 // g(x) = 1/x - 1/(x + tau)), and where a product underflows tau < 1e-153, so
-// that every measure is 1 beside eps = 1e-40. The measures are sums of squares:
-// their order is that of their bits, compared as integers off the FP64 pipe
-// (a NaN ends up in one of the products and fails the test).
+// that every measure is 1 beside eps = 1e-40. The ratio also grows with s_min
+// and falls with s_max, so a lower bound of the one and an upper bound of the
+// other are safe: the measures are sums of squares, ordered like their high
+// words, and the bounds are the least and greatest high word with the low word
+// all zeros or all ones (2^-20 of a value beside the 10% margin). That is two
+// three-way integer instructions in place of four FP64 comparisons. A NaN or an
+// infinity becomes a NaN in one of the products and fails the test.
 CFD_HD bool teno_z_all_kept(double s0, double s1, double s2, double tau, double kap)
 {
 #if defined(__CUDA_ARCH__)
-    const long long i0 = __double_as_longlong(s0), i1 = __double_as_longlong(s1), i2 = __double_as_longlong(s2);
-    const long long ia = i0 < i1 ? i0 : i1, ib = i0 < i1 ? i1 : i0;
-    const double smin = __longlong_as_double(ia < i2 ? ia : i2), smax = __longlong_as_double(ib < i2 ? i2 : ib);
+    const int h0 = __double2hiint(s0), h1 = __double2hiint(s1), h2 = __double2hiint(s2);
+    const double smin = __hiloint2double(__vimin3_s32(h0, h1, h2), 0);
+    const double smax = __hiloint2double(__vimax3_s32(h0, h1, h2), -1);
     const double lhs = (smax + tau) * smin, rhs = (smin + tau) * smax;
     // rhs < 2^996 (about 1e300), on the exponent bits
     return (__double2hiint(rhs) < (int)(2019u << 20)) & (lhs >= kap * rhs);
@@ -738,11 +788,16 @@ CFD_HD double inter5(double q0, double q1, double q2, double q3, double q4, doub
 #else
         double s;
         // (1/16) / s^2 = RN(1 / s^2) / 16 exactly (a power-of-two scaling)
-        s = eps + b0; b0 = o.rcp(s * s) * (1.0 / 16.0);
-        s = eps + b1; b1 = o.div_pos(5.0 / 8.0, s * s);
-        s = eps + b2; b2 = o.div_pos(5.0 / 16.0, s * s);
+        // (s^2 >= 1e-12; a negative or non-finite one fails need_below too)
+        s = eps + b0; const double s0 = s * s;
+        s = eps + b1; const double s1 = s * s;
+        s = eps + b2; const double s2 = s * s;
+        o.need_below(s0, s1, s2);
+        b0 = o.rcp_in(s0) * (1.0 / 16.0);
+        b1 = o.div_in(5.0 / 8.0, s1);
+        b2 = o.div_in(5.0 / 16.0, s2);
         const double sumbeta = b0 + b1 + b2, result = b0 * u0 + b1 * u1 + b2 * u2;
-        return o.div(result, sumbeta);
+        return o.div_b_in(result, sumbeta);
 #endif
     } else if constexpr (FAM == FAM_WENOZ) {
         // weno5_Z: omega_k = gamma_k (1 + (tau / (beta_k + eps))^2), eps = 1e-40.
@@ -1113,22 +1168,28 @@ CFD_HD double char_cons_to_prim(const double *cs, double *p, O &o)
     } else if constexpr (NV == 4) {
         double rt = cs[0], rut = cs[1], rvt = cs[2], ret = cs[3];
         const double irt = o.rcp(rt);
-        double ut = o.div_y(rut, rt, irt), vt = o.div_y(rvt, rt, irt);
+#if !defined(CFD_FAST)
+        o.need_sq(rut); o.need_sq(rvt);
+#endif
+        double ut = o.div_y_in(rut, rt, irt), vt = o.div_y_in(rvt, rt, irt);
 #if defined(CFD_FAST)
         double rekt = (rut * rut + rvt * rvt) * (0.5 * irt);
 #else
-        double rekt = o.div_y(rut * rut + rvt * rvt, rt, irt) / 2;
+        double rekt = o.div_y_in(rut * rut + rvt * rvt, rt, irt) / 2;
 #endif
         p[0] = rt; p[1] = ut; p[2] = vt; p[3] = (gamma - 1) * (ret - rekt);
         return irt;
     } else {
         double rt = cs[0], rut = cs[1], rvt = cs[2], rwt = cs[3], ret = cs[4];
         const double irt = o.rcp(rt);
-        double ut = o.div_y(rut, rt, irt), vt = o.div_y(rvt, rt, irt), wt = o.div_y(rwt, rt, irt);
+#if !defined(CFD_FAST)
+        o.need_sq(rut); o.need_sq(rvt); o.need_sq(rwt);
+#endif
+        double ut = o.div_y_in(rut, rt, irt), vt = o.div_y_in(rvt, rt, irt), wt = o.div_y_in(rwt, rt, irt);
 #if defined(CFD_FAST)
         double rekt = (rut * rut + rvt * rvt + rwt * rwt) * (0.5 * irt);
 #else
-        double rekt = o.div_y(rut * rut + rvt * rvt + rwt * rwt, rt, irt) / 2;
+        double rekt = o.div_y_in(rut * rut + rvt * rvt + rwt * rwt, rt, irt) / 2;
 #endif
         p[0] = rt; p[1] = ut; p[2] = vt; p[3] = wt; p[4] = (gamma - 1) * (ret - rekt);
         return irt;
@@ -1339,8 +1400,9 @@ struct EigenBase {
         const double coef = r * ir;
         k[E] = 0.5 * (coef * q2) + kG1 * (pp * ir);
 #else
-        const double coef = o.sqrt(r);
-        const double H = q2 / 2 + o.div_y(o.div_y(pp, r, irho) * kGamma, kGm1, kRcpGm1);
+        const double coef = o.sqrt_in(r);  // rho was checked for irho
+        o.need_pos(pp);
+        const double H = q2 / 2 + o.div_y_in(o.div_y_in(pp, r, irho) * kGamma, kGm1, kRcpGm1);
         k[E] = coef * H;
 #endif
         k[0] = coef;
@@ -1370,14 +1432,18 @@ struct EigenBase {
         c = c2 * ic;
         ih = (gamma - 1) * (ic * ic);
 #else
-        c = o.sqrt((gamma - 1) * h);
-        ic = o.rcp(c);
-        ih = o.rcp(h);
-        Vc = o.div_y(Vn, c, ic);
-        ekh = o.div_y(ek, h, ih);
-        uh = o.div_y(u, h, ih);
-        vh = o.div_y(v, h, ih);
-        wh = (D == 3) ? o.div_y(w, h, ih) : 0.0;
+        // one check of h and of each velocity covers c, Vn and ek
+        o.need_pos(h);
+        o.need_sq(u); o.need_sq(v);
+        if constexpr (D == 3) o.need_sq(w);
+        c = o.sqrt_in((gamma - 1) * h);
+        ic = o.rcp_in(c);
+        ih = o.rcp_in(h);
+        Vc = o.div_y_in(Vn, c, ic);
+        ekh = o.div_y_in(ek, h, ih);
+        uh = o.div_y_in(u, h, ih);
+        vh = o.div_y_in(v, h, ih);
+        wh = (D == 3) ? o.div_y_in(w, h, ih) : 0.0;
 #endif
     }
 
@@ -1697,10 +1763,12 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const d
     double VnL = vl[AX], VnR = vr[AX];
     double cl = o.sqrt(prl * gamma), cr = o.sqrt(prr * gamma);
 #else
-    const double prl = O::spec ? o.div_y(pl, rl, ir[0]) : pl / rl, prr = O::spec ? o.div_y(pr, rr, ir[1]) : pr / rr;
+    o.need_pos(pl);  // p in range (rho is: ir) covers p/rho and its multiples
+    o.need_pos(pr);
+    const double prl = O::spec ? o.div_y_in(pl, rl, ir[0]) : pl / rl, prr = O::spec ? o.div_y_in(pr, rr, ir[1]) : pr / rr;
     // x / (gamma - 1) by its correctly rounded reciprocal
     {
-        const double qq[2] = {o.div_y(prl * kGamma, kGm1, kRcpGm1), o.div_y(prr * kGamma, kGm1, kRcpGm1)};
+        const double qq[2] = {o.div_y_in(prl * kGamma, kGm1, kRcpGm1), o.div_y_in(prr * kGamma, kGm1, kRcpGm1)};
         if constexpr (D == 2) {
             HL = (vl[0] * vl[0] + vl[1] * vl[1]) / 2 + qq[0];
             HR = (vr[0] * vr[0] + vr[1] * vr[1]) / 2 + qq[1];
@@ -1710,7 +1778,7 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const d
         }
     }
     double VnL = vl[AX], VnR = vr[AX];
-    double cl = o.sqrt(prl * gamma), cr = o.sqrt(prr * gamma);
+    double cl = o.sqrt_in(prl * gamma), cr = o.sqrt_in(prr * gamma);
 #endif
     (void)ir;
     double rBar = (rl + rr) / 2, cBar = (cl + cr) / 2;
@@ -1718,8 +1786,15 @@ CFD_HD void hllc_md(const double *L, const double *R, double *res, O &o, const d
     double ps = (0.0 < ps0) ? ps0 : 0.0;  // std::max(0.0, .)
     double ql, qr;
     if constexpr (O::spec) {
-        const double tl = o.sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (o.div(ps, pl) - 1.0));
-        const double tr = o.sqrt(1.0 + (gamma + 1.0) / (2.0 * gamma) * (o.div(ps, pr) - 1.0));
+        // ps < 2^200 and p >= 2^-400 keep the quotient finite, its root is of a
+        // number above 1/7 (ps >= 0); a quotient below 2^-800 only meets 1.0
+#if defined(CFD_FAST)
+        o.need_pos(pl);
+        o.need_pos(pr);
+#endif
+        o.need_below(ps, ps, ps);
+        const double tl = o.sqrt_in(1.0 + (gamma + 1.0) / (2.0 * gamma) * (o.div_in(ps, pl) - 1.0));
+        const double tr = o.sqrt_in(1.0 + (gamma + 1.0) / (2.0 * gamma) * (o.div_in(ps, pr) - 1.0));
         ql = (ps <= pl) ? 1.0 : tl;
         qr = (ps <= pr) ? 1.0 : tr;
     } else {
@@ -1881,8 +1956,10 @@ CFD_HD void roe_md(const double *L, const double *R, double *res, O &o, const do
     double HL, HR;
     // x / (gamma - 1) by its correctly rounded reciprocal
     {
-        const double prl = O::spec ? o.div_y(pl, rl, ir[0]) : pl / rl, prr = O::spec ? o.div_y(pr, rr, ir[1]) : pr / rr;
-        const double qq[2] = {o.div_y(prl * kGamma, kGm1, kRcpGm1), o.div_y(prr * kGamma, kGm1, kRcpGm1)};
+        o.need_pos(pl);  // p in range (rho is: ir) covers p/rho and its multiples
+        o.need_pos(pr);
+        const double prl = O::spec ? o.div_y_in(pl, rl, ir[0]) : pl / rl, prr = O::spec ? o.div_y_in(pr, rr, ir[1]) : pr / rr;
+        const double qq[2] = {o.div_y_in(prl * kGamma, kGm1, kRcpGm1), o.div_y_in(prr * kGamma, kGm1, kRcpGm1)};
         if constexpr (D == 2) {
             HL = (vl[0] * vl[0] + vl[1] * vl[1]) / 2 + qq[0];
             HR = (vr[0] * vr[0] + vr[1] * vr[1]) / 2 + qq[1];
@@ -1900,9 +1977,9 @@ CFD_HD void roe_md(const double *L, const double *R, double *res, O &o, const do
     for (int i = 0; i < D; i++) FcR[1 + i] = (i == AX) ? rr * vr[i] * VnR + pr : rr * vr[i] * VnR;
     FcR[E] = rr * HR * VnR;
 
-    double coef1 = o.sqrt(rl), coef2 = o.sqrt(rr);
-    double divisor = o.rcp(coef1 + coef2);
-    double rhoAvg = o.sqrt(rl * rr);
+    double coef1 = o.sqrt_in(rl), coef2 = o.sqrt_in(rr);
+    double divisor = o.rcp_in(coef1 + coef2);
+    double rhoAvg = o.sqrt_in(rl * rr);
     double vAvg[3];
     for (int i = 0; i < D; i++) vAvg[i] = (coef1 * vl[i] + coef2 * vr[i]) * divisor;
     double HAvg = (coef1 * HL + coef2 * HR) * divisor;
@@ -1934,7 +2011,7 @@ CFD_HD void roe_md(const double *L, const double *R, double *res, O &o, const do
     double Fd[NV];
     // the three quotients by c^2 and 2 c^2 from one correctly rounded
     // reciprocal: (2 c) c = 2 RN(c c) exactly, so x / (2 c c) = RN(x / (c c)) / 2
-    const double cc2 = cAvg * cAvg, icc2 = o.rcp(cc2);
+    const double cc2 = cAvg * cAvg, icc2 = o.rcp_in(cc2);
     const double qc[3] = {o.div_y(deltaP - rhoAvg * cAvg * deltaVn, cc2, icc2),
                           o.div_y(deltaP + rhoAvg * cAvg * deltaVn, cc2, icc2), o.div_y(deltaP, cc2, icc2)};
     double c1 = qc[0] / 2;
