@@ -481,7 +481,7 @@ def batch_throughput(device, stream, ncases=256, steps=20, seed=0, full_run=True
         return e0.elapsed_time(e1), float(sum(n * n * int(k) for n, k in zip(sizes, ns))), ns
 
     b.run(0.25, end_step=1, max_steps=3)  # warm-up (graph capture)
-    ms0, cs0, _ = timed_run(steps)  # the default tiling: whole lines, single-grid tile shapes
+    ms0, cs0, _ = timed_run(steps)  # the default tiling
     tiling = b.autotune()
     b.run(0.25, end_step=1, max_steps=3)  # warm-up after the tiling change
     ms, cell_steps, _ = timed_run(steps)

@@ -1693,8 +1693,8 @@ struct cfd_batch {
     // CTAs take the longest tiles first and the tail holds the short ones
     std::vector<int> order;
     // tiling per direction, chosen by cfd_batch_autotune: tile shape (0 the
-    // single-grid shape, 1 the alternative), segments per line, one persistent
-    // CTA per SM instead of as many as fit
+    // single-grid shape, 1 the alternative), segments per line (at first
+    // batch_default_split), one persistent CTA per SM instead of as many as fit
     int shape[3] = {0, 0, 0}, split[3] = {1, 1, 1}, one_cta[3] = {0, 0, 0};
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
@@ -1746,8 +1746,47 @@ SweepParams batch_params(cfd_batch *b, int c, int slot, int stage, int d)
 int batch_chunk(const cfd_batch *b, int d)
 {
     if (b->nv == 3) return cfd::k1S;
-    if (d == 0) return b->shape[0] ? cfd::kXS2 : cfd::kXS;
-    return b->shape[d] ? cfd::kYS2 : cfd::kYS;
+    if (d == 0) return (b->shape[0] || (b->nv == 4 && b->prec)) ? cfd::kXS : cfd::kXSn;
+    return b->shape[d] ? cfd::kYS : cfd::kYSm;
+}
+
+// Lines per CTA of the same sweep.
+int batch_lines(const cfd_batch *b, int d)
+{
+    if (b->nv == 3) return cfd::k1W;
+    if (d == 0) return (b->shape[0] || (b->nv == 4 && b->prec)) ? cfd::kXW : cfd::kXWn;
+    return b->shape[d] ? cfd::kYW : cfd::kYWm;
+}
+
+// Segments per line the batch starts with along d: the least of all CTAs'
+// chunks over the resident CTAs (three per SM; each tile pays 0.85 of a chunk
+// for its second pass and set-up) plus half the longest tile, which the last
+// wave waits for. Whole lines left 24 grids of 128^2 to 512^2 two tiles a CTA
+// of up to 32 chunks.
+int batch_default_split(const cfd_batch *b, int d)
+{
+    const int S = batch_chunk(b, d), W = batch_lines(b, d);
+    int t0, t1, best = 1;
+    transverse_axes(d, t0, t1);
+    double best_cost = 1e300;
+    for (int split = 1; split <= 16; split *= 2) {
+        double work = 0.0, longest = 0.0;
+        for (const cfd_handle *h : b->h) {
+            const int n = h->cfg.n[d];
+            int seg = (n + split - 1) / split;
+            seg = std::min(n, (seg + S - 1) / S * S);
+            const double lines = (double)((h->cfg.n[t0] + W - 1) / W) * h->cfg.n[t1];
+            const double nseg = (n + seg - 1) / seg, chunks = (n + S - 1) / S;
+            work += lines * (chunks + 0.85 * nseg);
+            longest = std::max(longest, (double)((seg + S - 1) / S) + 0.85);
+        }
+        const double cost = std::max(work / (3.0 * b->num_sms) + 0.5 * longest, longest);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = split;
+        }
+    }
+    return best;
 }
 
 // Segment lengths of every case (lines cut into split[d] segments of whole
@@ -1870,8 +1909,8 @@ int cfd_batch_create(const cfd_config *cfgs, int ncases, cfd_batch **out)
     b->order.resize(ncases);
     for (int c = 0; c < ncases; c++) b->order[c] = c;
     std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) { return b->h[x]->ncell > b->h[y]->ncell; });
-    // whole lines by default (cfd_batch_autotune may cut them); the config's
-    // seg_len of each case is replaced by the batch's tiling
+    // the config's seg_len of each case is replaced by the batch's tiling
+    for (int d = 0; d < b->dim; d++) b->split[d] = batch_default_split(b, d);
     if ((e = cudaMalloc(&b->d_tile_start, sizeof(long long) * b->dim * (ncases + 1))) != cudaSuccess) return bail(e);
     int rc = batch_layout(b);
     if (rc) {
@@ -2041,7 +2080,7 @@ int cfd_batch_autotune(cfd_batch *b, int *choice, double *ms)
         float best = 3.4e38f;
         int best_cfg[3] = {b->shape[d], b->split[d], b->one_cta[d]};
         for (int shape = 0; shape <= (alt ? 1 : 0) && rc == CFD_OK; shape++)
-            for (int split = 1; split <= 2 && rc == CFD_OK; split++)
+            for (int split = 1; split <= 8 && rc == CFD_OK; split *= 2)
                 for (int one = 0; one <= 1 && rc == CFD_OK; one++) {
                     b->shape[d] = shape;
                     b->split[d] = split;

@@ -845,16 +845,6 @@ static cudaError_t launch_batched_shape_p(const BatchSweep &b, cudaStream_t st)
     return cudaGetLastError();
 }
 
-template <int NV, int AX, int FAM, int FLUX, int S, int W>
-static cudaError_t launch_batched_shape(const BatchSweep &b, cudaStream_t st)
-{
-    if (b.prec == 0) return launch_batched_shape_p<NV, AX, FAM, FLUX, S, W, 0>(b, st);
-#if defined(CFD_FAST)
-    if constexpr (NV >= 4 && FAM != FAM_RESEARCH) return launch_batched_shape_p<NV, AX, FAM, FLUX, S, W, 1>(b, st);
-#endif
-    return cudaErrorInvalidValue;
-}
-
 // FP64 or, in the fast flavour of the multi-dimensional kernels, mixed; the
 // TRAD6 difference in FP64 only.
 template <int NV, int AX, int FAM, int FLUX, int S, int W>
@@ -870,9 +860,8 @@ static cudaError_t launch_sweep_shape(const SweepParams &p, cudaStream_t st)
 }
 
 // Tile shapes (sweep_params.h): kXSn x kXWn along x in 3D and for 2D FP64,
-// kXS x kXW along x for the 2D mixed form; kYSm x kYWm along y and z for the
-// single-grid sweeps; kXS x kXW and kYS x kYW for the TRAD6 difference and the
-// batched kernel's default; k1S x k1W in 1D.
+// kXS x kXW along x for the 2D mixed form; kYSm x kYWm along y and z;
+// kXS x kXW and kYS x kYW for the TRAD6 difference; k1S x k1W in 1D.
 template <int NV, int FAM>
 cudaError_t launch_sweep(int ax, int flux, const SweepParams &p, cudaStream_t st)
 {
@@ -929,41 +918,48 @@ cudaError_t launch_sweep(int ax, int flux, const SweepParams &p, cudaStream_t st
     }
 }
 
-// Persistent batched sweep (1D, 2D and 3D; the tile shapes of launch_sweep or,
-// for 2D/3D FP64 with b.shape = 1, the alternative shapes).
+// Persistent batched sweep (1D, 2D and 3D): the single-grid tile shapes, or for
+// 2D/3D FP64 with b.shape = 1 the alternatives.
+template <int NV, int AX, int FAM, int S, int W, int PREC>
+static cudaError_t launch_batched_flux(int flux, const BatchSweep &b, cudaStream_t st)
+{
+    return flux == FLUX_HLLC ? launch_batched_shape_p<NV, AX, FAM, FLUX_HLLC, S, W, PREC>(b, st)
+                             : launch_batched_shape_p<NV, AX, FAM, FLUX_ROE, S, W, PREC>(b, st);
+}
+
+template <int NV, int AX, int FAM>
+static cudaError_t launch_batched_ax(int flux, const BatchSweep &b, cudaStream_t st)
+{
+    if (b.prec == 1) {
+#if defined(CFD_FAST)
+        if constexpr (FAM != FAM_RESEARCH) {
+            if (b.shape) return cudaErrorInvalidValue;
+            if constexpr (AX == 0 && NV == 4) return launch_batched_flux<NV, AX, FAM, kXS, kXW, 1>(flux, b, st);
+            else if constexpr (AX == 0) return launch_batched_flux<NV, AX, FAM, kXSn, kXWn, 1>(flux, b, st);
+            else return launch_batched_flux<NV, AX, FAM, kYSm, kYWm, 1>(flux, b, st);
+        }
+#endif
+        return cudaErrorInvalidValue;
+    }
+    if constexpr (AX == 0)
+        return b.shape ? launch_batched_flux<NV, AX, FAM, kXS, kXW, 0>(flux, b, st)
+                       : launch_batched_flux<NV, AX, FAM, kXSn, kXWn, 0>(flux, b, st);
+    else
+        return b.shape ? launch_batched_flux<NV, AX, FAM, kYS, kYW, 0>(flux, b, st)
+                       : launch_batched_flux<NV, AX, FAM, kYSm, kYWm, 0>(flux, b, st);
+}
+
 template <int NV, int FAM>
 cudaError_t launch_sweep_batched(int ax, int flux, const BatchSweep &b, cudaStream_t st)
 {
     if constexpr (NV == 3) {
-        if (ax != 0) return cudaErrorInvalidValue;
-        return flux == FLUX_HLLC ? launch_batched_shape<3, 0, FAM, FLUX_HLLC, k1S, k1W>(b, st)
-                                 : launch_batched_shape<3, 0, FAM, FLUX_ROE, k1S, k1W>(b, st);
+        if (ax != 0 || b.prec != 0) return cudaErrorInvalidValue;
+        return launch_batched_flux<3, 0, FAM, k1S, k1W, 0>(flux, b, st);
     } else {
-        if (b.shape == 1) {
-            if (b.prec != 0) return cudaErrorInvalidValue;
-            if (ax == 0)
-                return flux == FLUX_HLLC ? launch_batched_shape_p<NV, 0, FAM, FLUX_HLLC, kXS2, kXW2, 0>(b, st)
-                                         : launch_batched_shape_p<NV, 0, FAM, FLUX_ROE, kXS2, kXW2, 0>(b, st);
-            if (ax == 1)
-                return flux == FLUX_HLLC ? launch_batched_shape_p<NV, 1, FAM, FLUX_HLLC, kYS2, kYW2, 0>(b, st)
-                                         : launch_batched_shape_p<NV, 1, FAM, FLUX_ROE, kYS2, kYW2, 0>(b, st);
-            if constexpr (NV == 5) {
-                if (ax == 2)
-                    return flux == FLUX_HLLC ? launch_batched_shape_p<NV, 2, FAM, FLUX_HLLC, kYS2, kYW2, 0>(b, st)
-                                             : launch_batched_shape_p<NV, 2, FAM, FLUX_ROE, kYS2, kYW2, 0>(b, st);
-            }
-            return cudaErrorInvalidValue;
-        }
-        if (ax == 0)
-            return flux == FLUX_HLLC ? launch_batched_shape<NV, 0, FAM, FLUX_HLLC, kXS, kXW>(b, st)
-                                     : launch_batched_shape<NV, 0, FAM, FLUX_ROE, kXS, kXW>(b, st);
-        if (ax == 1)
-            return flux == FLUX_HLLC ? launch_batched_shape<NV, 1, FAM, FLUX_HLLC, kYS, kYW>(b, st)
-                                     : launch_batched_shape<NV, 1, FAM, FLUX_ROE, kYS, kYW>(b, st);
+        if (ax == 0) return launch_batched_ax<NV, 0, FAM>(flux, b, st);
+        if (ax == 1) return launch_batched_ax<NV, 1, FAM>(flux, b, st);
         if constexpr (NV == 5) {
-            if (ax == 2)
-                return flux == FLUX_HLLC ? launch_batched_shape<NV, 2, FAM, FLUX_HLLC, kYS, kYW>(b, st)
-                                         : launch_batched_shape<NV, 2, FAM, FLUX_ROE, kYS, kYW>(b, st);
+            if (ax == 2) return launch_batched_ax<NV, 2, FAM>(flux, b, st);
         }
         return cudaErrorInvalidValue;
     }

@@ -7,7 +7,7 @@ namespace cfd {
 // Tile shapes of the sweeps: cells per chunk (S) x lines per CTA (W). CTAs of
 // 128 threads run three or four per SM (barriers across 4 warps instead of 8):
 // every 2D/3D sweep takes them; the 32-line shapes (256 threads) remain for
-// the batched kernel and the TRAD6 difference.
+// the TRAD6 difference and as the batched kernel's alternative.
 #ifndef CFD_XS
 #define CFD_XS 32
 #endif
@@ -20,16 +20,16 @@ namespace cfd {
 #ifndef CFD_YW
 #define CFD_YW 32
 #endif
-constexpr int kXS = CFD_XS, kXW = CFD_XW;  // along x (2D mixed, TRAD6, batched default)
-constexpr int kXSn = 16, kXWn = 8;          // along x: 3D, and 2D FP64 (single grid)
-constexpr int kYS = CFD_YS, kYW = CFD_YW;  // along y and z
+constexpr int kXS = CFD_XS, kXW = CFD_XW;  // along x (2D mixed, TRAD6, batched alternative)
+constexpr int kXSn = 16, kXWn = 8;          // along x: 3D, and 2D FP64
+constexpr int kYS = CFD_YS, kYW = CFD_YW;  // along y and z (TRAD6, batched alternative)
 #ifndef CFD_YSM
 #define CFD_YSM 8
 #endif
 #ifndef CFD_YWM
 #define CFD_YWM 16
 #endif
-constexpr int kYSm = CFD_YSM, kYWm = CFD_YWM;  // along y, mixed form (single grid)
+constexpr int kYSm = CFD_YSM, kYWm = CFD_YWM;  // along y and z
 #ifndef CFD_FP64_3D_YZ16
 #define CFD_FP64_3D_YZ16 1  // the FP64 3D y/z sweeps take the kYSm x kYWm shape too (0: kYS x kYW)
 #endif
@@ -40,11 +40,6 @@ constexpr int kYSm = CFD_YSM, kYWm = CFD_YWM;  // along y, mixed form (single gr
 #define CFD_MIXED_Z16 1  // the mixed form's z sweep takes the kYSm x kYWm shape too (0: kYS x kYW)
 #endif
 constexpr int k1S = 128, k1W = 1;          // 1D
-// Alternative shapes of the batched 2D/3D FP64 sweeps, picked per direction by
-// the batch autotuner: 32 threads per x line (8 lines per CTA), 8 threads per
-// y/z line (16 lines per CTA, the single-grid FP64 shape).
-constexpr int kXS2 = 32, kXW2 = 8;
-constexpr int kYS2 = 8, kYW2 = 16;
 
 
 // BndType values (zone_FD/src/include/macro.hpp:33-34) plus the 3D mirror.
@@ -143,7 +138,7 @@ struct BatchSweep {
     long long total_tiles;
     int num_sms;
     int prec;
-    int shape;      // 0: default tile shape, 1: the alternative (kXS2 x kXW2 / kYS2 x kYW2; 2D/3D FP64 only)
+    int shape;      // 0: the single-grid tile shapes, 1: the alternative (kXS x kXW / kYS x kYW; 2D/3D FP64 only)
     int one_cta;    // 1: one persistent CTA per SM, 0: as many as fit
 };
 
