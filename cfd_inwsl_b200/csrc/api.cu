@@ -87,46 +87,16 @@ __global__ void __launch_bounds__(256) wave_speed_kernel(const double *__restric
     cfd::block_max_reduce<256, 4>(0.0, lam, red);
 }
 
-// Step control of stepsLoopCFL (blockSolver.cpp:176-201) on the device: the
-// loop test, dt = CFL / sum_d lambda_d from the wave-speed maxima of the
-// current state, clipping to the output interval, stage coefficients.
+// The step control (sweep_params.h) as kernels of their own, for steps whose
+// last sweep does not carry it.
 __global__ void step_begin_kernel(cfd::StepCtl *c, unsigned long long *red, int dim, double *dts)
 {
-    if (c->done) return;
-    if (!(c->step < c->endStep && c->k < c->maxSteps)) {
-        c->done = 1;
-        return;
-    }
-    double lambda = 0;
-    for (int d = 0; d < dim; d++) lambda += __longlong_as_double((long long)red[1 + d]);
-    double dt = c->cfl / lambda;
-    if (c->outputT + dt > c->outputDt) {
-        dt = c->outputDt - c->outputT;
-        c->outputT = 0.0;
-        c->step++;
-    } else
-        c->outputT += dt;
-    c->dt = dt;
-    c->bdt[1] = dt;
-    c->bdt[2] = 0.25 * dt;
-    c->bdt[3] = 2.0 / 3.0 * dt;
-    c->tst[1] = c->t;
-    c->tst[2] = c->t + dt;
-    c->tst[3] = c->tst[2] - dt / 2;
-    if (dts) dts[c->k] = dt;
-    // the wave speeds are consumed: clear the reduction words for this step's
-    // third stage (only when the step runs, so a finished loop keeps them)
-    for (int i = 0; i < 4; i++) red[i] = 0ULL;
+    cfd::step_begin(c, red, dim, dts);
 }
 
-// BlockSolver::solve's time update and the per-step log value (rhoLinf).
 __global__ void step_end_kernel(cfd::StepCtl *c, const unsigned long long *red, double *linf)
 {
-    if (c->done) return;
-    if (linf) linf[c->k] = __longlong_as_double((long long)red[0]);
-    double dt = c->dt;
-    c->t = (((c->t + dt) - dt / 2) - dt / 2) + dt;
-    c->k++;
+    cfd::step_end(c, red, linf);
 }
 
 // FP64 peak probe: eight independent DFMA chains per thread over every SM,
@@ -406,6 +376,7 @@ struct cfd_handle {
     double *stage = nullptr;  // AoS staging buffer
     unsigned long long *red = nullptr;
     unsigned *err = nullptr;
+    unsigned *ticket = nullptr;  // finished CTAs of a step's last sweep (beside err; 0 between launches)
     std::vector<BcLine> bc_lo[3], bc_hi[3];
     std::vector<double> bc_vals;
     BcLine *d_bclo[3] = {nullptr, nullptr, nullptr};
@@ -800,19 +771,23 @@ int ensure_run_buffers(cfd_handle *h, int max_steps)
     return CFD_OK;
 }
 
-// Enqueue one device-controlled SSP-RK3 step (buffers by role).
+// Enqueue one device-controlled SSP-RK3 step (buffers by role), begun by
+// step_begin_kernel or by the step before: the last CTA of its last sweep ends
+// it and begins the next.
 int enqueue_step(cfd_handle *h, int cur)
 {
     double *U0 = h->u[cur], *U1 = h->u[(cur + 1) % 3], *U2 = h->u[(cur + 2) % 3];
-    step_begin_kernel<<<1, 1, 0, h->stream>>>(h->ctl, h->red, h->dim, h->d_dts);
-    CFD_CUDA(h, cudaGetLastError());
     int rc;
     if ((rc = rk_stage(h, 1, U0, U0, U1, 1.0, 0.0, 0.0, 0.0, false, h->ctl))) return rc;
     if ((rc = rk_stage(h, 2, U1, U0, U2, 0.75, 0.0, 0.25, 0.0, false, h->ctl))) return rc;
-    if ((rc = rk_stage(h, 3, U2, U0, U1, 1.0 / 3.0, 0.0, 2.0 / 3.0, 0.0, true, h->ctl))) return rc;
-    step_end_kernel<<<1, 1, 0, h->stream>>>(h->ctl, h->red, h->d_linf);
-    CFD_CUDA(h, cudaGetLastError());
-    return CFD_OK;
+    const int L = h->dim - 1;
+    if (L > 0 && (rc = rk_stage(h, 3, U2, U0, U1, 1.0 / 3.0, 0.0, 2.0 / 3.0, 0.0, true, h->ctl, 0, L))) return rc;
+    SweepParams p = stage_params(h, L, 3, U2, U0, U1, 1.0 / 3.0, 0.0, 2.0 / 3.0, 0.0, true, h->ctl);
+    p.ctl_step = h->ctl;
+    p.ticket = h->ticket;
+    p.dts = h->d_dts;
+    p.linf = h->d_linf;
+    return sweep(h, L, p);
 }
 
 // Capture kGraphSteps[gi] device-controlled steps starting at state slot
@@ -928,8 +903,9 @@ int cfd_create(const cfd_config *cfg, cfd_handle **out)
     if ((e = cudaMalloc(&h->rhs, bytes)) != cudaSuccess) return bail(e, "rhs");
     if ((e = cudaMalloc(&h->stage, bytes)) != cudaSuccess) return bail(e, "staging");
     if ((e = cudaMalloc(&h->red, 8 * sizeof(unsigned long long))) != cudaSuccess) return bail(e, "reductions");
-    if ((e = cudaMalloc(&h->err, sizeof(unsigned))) != cudaSuccess) return bail(e, "error word");
-    if ((e = cudaMemsetAsync(h->err, 0, sizeof(unsigned), h->stream)) != cudaSuccess) return bail(e, "memset");
+    if ((e = cudaMalloc(&h->err, 2 * sizeof(unsigned))) != cudaSuccess) return bail(e, "error word");
+    h->ticket = h->err + 1;
+    if ((e = cudaMemsetAsync(h->err, 0, 2 * sizeof(unsigned), h->stream)) != cudaSuccess) return bail(e, "memset");
     for (int k = 0; k < 3; k++)
         if ((e = cudaMemsetAsync(h->u[k], 0, bytes, h->stream)) != cudaSuccess) return bail(e, "memset");
     for (int d = 0; d < h->dim; d++) {
@@ -1135,14 +1111,17 @@ int cfd_run(cfd_handle *h, double cfl, int end_step, double output_dt, int max_s
     c->endStep = end_step;
     c->maxSteps = max_steps;
     CFD_CUDA(h, cudaMemcpyAsync(h->ctl, c, sizeof(*c), cudaMemcpyHostToDevice, h->stream));
-    CFD_CUDA(h, cudaMemsetAsync(h->err, 0, sizeof(unsigned), h->stream));
+    CFD_CUDA(h, cudaMemsetAsync(h->err, 0, 2 * sizeof(unsigned), h->stream));
+    step_begin_kernel<<<1, 1, 0, h->stream>>>(h->ctl, h->red, h->dim, h->d_dts);
+    CFD_CUDA(h, cudaGetLastError());
+    h->launches++;
     const int cur0 = h->cur;
     // Steps are launched as captured graphs of 12, 3 or 1 steps covering
     // exactly max_steps; if the output-interval test ends the loop earlier the
     // remaining launched steps are no-ops on the device. The host checks the
     // device state between batches whose size doubles.
     int launched = 0, slot = cur0, quota = 12;
-    const unsigned long long per_step = 2 + 3ULL * h->dim;
+    const unsigned long long per_step = 3ULL * h->dim;
     while (true) {
         int target = launched + quota;
         if (target > max_steps) target = max_steps;

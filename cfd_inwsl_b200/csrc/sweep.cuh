@@ -722,6 +722,18 @@ __global__ void __launch_bounds__(S *W, (SweepShape<NV, AX, FAM, FLUX, S, W, PRE
     sweep_kernel(const __grid_constant__ SweepParams p)
 {
     sweep_tile<NV, AX, FAM, FLUX, S, W, PREC, DIFF>(p, (int)(p.tile0 + blockIdx.x));
+    if constexpr (AX == NV - 3) {
+        if (p.ctl_step) {
+            __threadfence();  // this CTA's maxima before its ticket
+            __syncthreads();
+            if (threadIdx.x == 0 && atomicAdd(p.ticket, 1u) == gridDim.x - 1) {
+                __threadfence();
+                *p.ticket = 0u;
+                step_end(p.ctl_step, p.red, p.linf);
+                step_begin(p.ctl_step, p.red, NV - 2, p.dts);
+            }
+        }
+    }
 }
 
 // Number of CTA tiles one case's sweep along AX needs.

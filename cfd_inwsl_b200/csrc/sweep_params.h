@@ -87,6 +87,52 @@ struct StepCtl {
     int step, endStep, k, maxSteps, done, pad;
 };
 
+#if defined(__CUDACC__)
+// Step control of stepsLoopCFL (blockSolver.cpp:176-201) on the device: the
+// loop test, dt = CFL / sum_d lambda_d from the wave-speed maxima of the
+// current state, clipping to the output interval, stage coefficients.
+// (Products by powers of two only beside the sums, so that either flavour's
+// unit rounds it alike.)
+__device__ __forceinline__ void step_begin(StepCtl *c, unsigned long long *red, int dim, double *dts)
+{
+    if (c->done) return;
+    if (!(c->step < c->endStep && c->k < c->maxSteps)) {
+        c->done = 1;
+        return;
+    }
+    double lambda = 0;
+    for (int d = 0; d < dim; d++) lambda += __longlong_as_double((long long)__ldcg(red + 1 + d));
+    double dt = c->cfl / lambda;
+    if (c->outputT + dt > c->outputDt) {
+        dt = c->outputDt - c->outputT;
+        c->outputT = 0.0;
+        c->step++;
+    } else
+        c->outputT += dt;
+    c->dt = dt;
+    c->bdt[1] = dt;
+    c->bdt[2] = 0.25 * dt;
+    c->bdt[3] = 2.0 / 3.0 * dt;
+    c->tst[1] = c->t;
+    c->tst[2] = c->t + dt;
+    c->tst[3] = c->tst[2] - dt / 2;
+    if (dts) dts[c->k] = dt;
+    // the wave speeds are consumed: clear the reduction words for this step's
+    // third stage (only when the step runs, so a finished loop keeps them)
+    for (int i = 0; i < 4; i++) red[i] = 0ULL;
+}
+
+// BlockSolver::solve's time update and the per-step log value (rhoLinf).
+__device__ __forceinline__ void step_end(StepCtl *c, const unsigned long long *red, double *linf)
+{
+    if (c->done) return;
+    if (linf) linf[c->k] = __longlong_as_double((long long)__ldcg(red));
+    double dt = c->dt;
+    c->t = (((c->t + dt) - dt / 2) - dt / 2) + dt;
+    c->k++;
+}
+#endif
+
 struct SweepParams {
     const double *u;    // current state U_k, planar SoA u[v * ncell + cell]
     const double *u0;   // RK base state U_0
@@ -127,6 +173,13 @@ struct SweepParams {
     int part_lo, part_hi;
     int seg_outer;
     long long tile0;
+    // The last sweep of a device-controlled step (cfd_run): its last CTA ends
+    // the step and begins the next one, in place of two one-thread kernels
+    // between the steps (about 2.5 us each, a tenth of a small grid's step).
+    // ticket counts finished CTAs and is left at 0; null elsewhere.
+    StepCtl *ctl_step;
+    unsigned *ticket;
+    double *dts, *linf;
 };
 
 // One batched sweep launch: the parameter blocks of every case (device array)
