@@ -26,7 +26,7 @@ using cfd::BcLine;
 using cfd::SweepParams;
 
 namespace cfd {
-int default_seg_len_for(const cfd_config *cfg, int fam, bool strict, int d);
+int default_seg_len_for(const cfd_config *cfg, int d);
 bool config_bc_ok(const cfd_config *cfg, const char **why);
 }
 
@@ -674,7 +674,7 @@ int rk_stage(cfd_handle *h, int stage, const double *uin, const double *u0, doub
 
 int default_seg_len(const cfd_handle *h, int d)
 {
-    return cfd::default_seg_len_for(&h->cfg, h->fam, h->strict, d);
+    return cfd::default_seg_len_for(&h->cfg, d);
 }
 
 
@@ -1496,24 +1496,14 @@ namespace cfd {
 // Default cells per CTA segment along direction d for the tile shapes that
 // launch_sweep picks for this configuration. Shared with the allocation-free
 // entry point (noalloc.cu).
-int default_seg_len_for(const cfd_config *cfg, int fam, bool strict, int d)
+int default_seg_len_for(const cfd_config *cfg, int d)
 {
-    int n = cfg->n[d];
-    int S = (cfg->dim == 1) ? cfd::k1S : (d == 0 ? cfd::kXS : cfd::kYS);
-    int W = (cfg->dim == 1) ? cfd::k1W : (d == 0 ? cfd::kXW : cfd::kYW);
-    if (cfg->dim > 1 && d == 0 && cfg->diff_method != CFD_DIFF_TRAD6 &&
-        (cfg->dim == 3 || cfg->precision == CFD_PREC_FP64)) {
-        S = cfd::kXSn;  // the x sweep shape of launch_sweep
-        W = cfd::kXWn;
-    }
-    const bool mixed_shape = (d == 1 || (d == 2 && CFD_MIXED_Z16)) && cfg->precision == CFD_PREC_MIXED && !strict &&
-                             fam != cfd::FAM_RESEARCH;
-    const bool fp64_shape = cfg->precision == CFD_PREC_FP64 &&
-                            ((CFD_FP64_3D_YZ16 && cfg->dim == 3 && d > 0) || (CFD_FP64_2D_Y16 && cfg->dim == 2 && d == 1));
-    if (cfg->dim > 1 && (mixed_shape || fp64_shape) && cfg->diff_method != CFD_DIFF_TRAD6) {
-        S = cfd::kYSm;  // the mixed form's y sweep shape (launch_sweep)
-        W = cfd::kYWm;
-    }
+    const int n = cfg->n[d];
+    // the shapes of launch_sweep_ax
+    const bool trad6 = cfg->diff_method == CFD_DIFF_TRAD6;
+    const bool wide_x = trad6 || (cfg->dim == 2 && cfg->precision == CFD_PREC_MIXED);
+    const int S = (cfg->dim == 1) ? cfd::k1S : d == 0 ? (wide_x ? cfd::kXS : cfd::kXSn) : (trad6 ? cfd::kYS : cfd::kYSm);
+    const int W = (cfg->dim == 1) ? cfd::k1W : d == 0 ? (wide_x ? cfd::kXW : cfd::kXWn) : (trad6 ? cfd::kYW : cfd::kYWm);
     int t0, t1;
     transverse_axes(d, t0, t1);
     long long blocks_per_seg = (long long)((cfg->n[t0] + W - 1) / W) * cfg->n[t1];
@@ -1524,24 +1514,28 @@ int default_seg_len_for(const cfd_config *cfg, int fam, bool strict, int d)
     int seg = n;
     while (blocks_per_seg * ((n + seg - 1) / seg) < target && seg > 4 * S) seg = (seg + 1) / 2;
     if (blocks_per_seg * ((n + seg - 1) / seg) >= target) return seg;
-    // Grids too small for that: whole chunks per segment, by cost. A CTA's is
-    // its chunks, the first one's second pass over the extra faces (nearly a
-    // chunk's latency) and half a chunk of set-up, times its waves over 3
-    // resident CTAs per SM; below one wave a chunk takes about 4 us with one
-    // CTA per SM and hardly longer with three, so the longest CTA counts and
-    // one-chunk segments win; above it the mean counts, and a wave that is
-    // nearly empty costs about half a full one. Fitted on sweeps timed over 1
-    // to 64 chunks a segment from a 400-cell line to 512^2. Stopping at four
-    // chunks left a 64^2 grid 8 CTAs and a 400-cell line one: 24 strict steps
-    // of 64^2 4.10 -> 1.93 ms, 300 of 400 cells 31.3 -> 14.1 ms.
+    // Grids too small for that: one chunk of S - 3 cells (sweep_tile's ONE,
+    // strict flavour) or whole chunks per segment, by cost. A CTA's is its chunks, the second
+    // pass over the extra faces of longer segments (nearly a chunk's latency)
+    // and half a chunk of set-up, times its waves over 3 resident CTAs per SM;
+    // below one wave a chunk takes about as long with one CTA per SM as with
+    // three, so the longest CTA counts; above it the mean counts, and a wave
+    // that is nearly empty costs about half a full one. Fitted on sweeps timed
+    // over 1 to 64 chunks a segment from a 400-cell line to 512^2. Stopping at
+    // four chunks left a 64^2 grid 8 CTAs and a 400-cell line one: 24 strict
+    // steps of 64^2 4.10 -> 1.93 ms, 300 of 400 cells 31.3 -> 14.1 ms; the
+    // one-chunk kernel took them on from 1.51 to 1.22 and from 6.96 to 5.81 ms.
     double best = 1e300;
-    for (int s = S; ; s += S) {
+    const bool one = cfg->strict && !trad6;
+    for (int s = one ? S - 3 : S; ; s += (s % S) ? 3 : S) {
         const int len = s < n ? s : n;
         const long long nseg = (n + len - 1) / len;
         const int tail = n - (int)(nseg - 1) * len;
+        const double pass2 = (one && len <= S - 3) ? 0.0 : 1.0;
         const double k = (len + S - 1) / S, w = (double)(blocks_per_seg * nseg) / (148.0 * 3);
         const double mean = ((double)(nseg - 1) * k + (tail + S - 1) / S) / (double)nseg;
-        const double cost = w <= 1.0 ? (k + 1.3) * (0.85 + 0.3 * w) : (mean + 0.85) * (0.5 * (std::ceil(w) + w) + 0.3);
+        const double cost = w <= 1.0 ? (k + 0.4 + 0.9 * pass2) * (0.85 + 0.3 * w)
+                                     : (mean + 0.5 + 0.35 * pass2) * (0.5 * (std::ceil(w) + w) + 0.3);
         if (cost < best) {
             best = cost;
             seg = len;

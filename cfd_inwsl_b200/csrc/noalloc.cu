@@ -19,7 +19,7 @@
 
 namespace cfd {
 bool map_inter_method_for(int inter_method, int dim, int *fam, double *c);
-int default_seg_len_for(const cfd_config *cfg, int fam, bool strict, int d);
+int default_seg_len_for(const cfd_config *cfg, int d);
 bool config_bc_ok(const cfd_config *cfg, const char **why);
 }
 
@@ -203,7 +203,7 @@ extern "C" int cfd_rhs_noalloc(const cfd_config *cfg, const double *cons_soa, do
         p.t = t;
         p.icst = icst;
         p.icst_k = (fam == cfd::FAM_TENOZ) ? cfd::teno_kappa(icst) : 0.0;
-        p.seg_len = cfg->seg_len[d] > 0 ? cfg->seg_len[d] : cfd::default_seg_len_for(cfg, fam, cfg->strict != 0, d);
+        p.seg_len = cfg->seg_len[d] > 0 ? cfg->seg_len[d] : cfd::default_seg_len_for(cfg, d);
         p.dm_u = 8.25 * std::cos(M_PI / 6);
         p.dm_v = -8.25 * std::sin(M_PI / 6);
         p.gravity = (cfg->source_type == 1 && d == cfg->dim - 1) ? 1 : 0;

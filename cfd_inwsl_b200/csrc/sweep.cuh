@@ -278,8 +278,7 @@ struct SweepShape {
     // fast flavour: 3.35 -> 3.23 and 1.90 -> 1.78 ms per 256^3 launch at
     // three CTAs), the FP64 TENO-Z x sweep and the 3D mixed TENO-Z sweeps.
     static constexpr bool THREE = ((FAM == FAM_TENOZ) && (PREC == 0 ? AX == 0 : NV == 5)) ||
-                                  (CFD_FP64_3D_YZ16 && PREC == 0 && NV == 5) ||
-                                  (CFD_FP64_2D_Y16 && PREC == 0 && NV == 4 && AX == 1);
+                                  (PREC == 0 && NV == 5) || (PREC == 0 && NV == 4 && AX == 1);
     // The strict flavour's 3D z sweep (the stage-closing one) measured 7%
     // faster at two CTAs per SM (255 registers) than at three.
     static constexpr bool TWO = kStrictFlavour && PREC == 0 && NV == 5 && AX == 2;
@@ -309,7 +308,13 @@ struct SweepShape {
     static constexpr size_t SMEM_BYTES = SMEM_RINGS + (PF ? SMEM_STAGE : 0);
 };
 
-template <int NV, int AX, int FAM, int FLUX, int S, int W, int PREC, int DIFF>
+// ONE: every segment has at most S - FC cells. Its faces are one pass of the
+// threads: the prologue loads HG + 2 - FO cells and the chunk S, and the cells
+// are finished by the threads from FC on. Otherwise a segment's first chunk
+// takes the FC faces ahead of it in a second pass, nearly another face's
+// latency, which long segments spread over their chunks. (One kernel for both
+// lengths cost the long ones 5 to 14%: the offsets became variables.)
+template <int NV, int AX, int FAM, int FLUX, int S, int W, int PREC, int DIFF, bool ONE = false>
 __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
 {
     using SH = SweepShape<NV, AX, FAM, FLUX, S, W, PREC, DIFF>;
@@ -503,10 +508,11 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
         for (int v = 0; v < NV; v++) sf[(v * W + l) * LSF + fslot] = fx[v];
     };
 
-    // prologue: cells s_begin-HG .. s_begin+HG-1
-    for (int idx = tid; idx < 2 * HG * W; idx += NT) {
-        int l = (AX == 0) ? idx / (2 * HG) : idx % W;
-        int q = (AX == 0) ? idx % (2 * HG) : idx / W;
+    // prologue: cells s_begin-HG .. s_begin+HC-1, HC of the chunks' offset
+    constexpr int HC = ONE ? 2 - FO : HG;
+    for (int idx = tid; idx < (HG + HC) * W; idx += NT) {
+        int l = (AX == 0) ? idx / (HG + HC) : idx % W;
+        int q = (AX == 0) ? idx % (HG + HC) : idx / W;
         load_pos(l, s_begin - HG + q);
     }
 
@@ -530,7 +536,7 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
     auto prefetch_epilogue = [&](int i) {
         bool ok; long long base; int lid;
         own_line(ok, base, lid);
-        if (ok && i < s_end) {
+        if (ok && i < s_end && (!ONE || i >= s_begin)) {
             const long long cell = base + (long long)i * sAX;
 #pragma unroll
             for (int v = 0; v < NV; v++) {
@@ -542,10 +548,17 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
         }
         __pipeline_commit();
     };
-    if constexpr (PF) prefetch_cell(s_begin + HG + tp);
+    if constexpr (ONE) {
+        // the epilogue's operands fly while the faces are computed
+        if constexpr (PF) prefetch_epilogue(s_begin - FC + tp);
+    } else if constexpr (PF) {
+        prefetch_cell(s_begin + HG + tp);
+    }
 
-    for (int c0 = s_begin; c0 < s_end; c0 += S) {
-        if constexpr (PF) {
+    for (int c0 = s_begin; ONE ? c0 == s_begin : c0 < s_end; c0 += S) {
+        if constexpr (ONE) {
+            if (tp < s_end - s_begin + FC) load_pos(tl, c0 + HC + tp);
+        } else if constexpr (PF) {
             __pipeline_wait_prior(0);
             load_pos(tl, c0 + HG + tp, true);
             prefetch_epilogue(c0 + tp);
@@ -558,12 +571,12 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
             // the chunk's S new faces per line, and before the segment's first
             // chunk also the FC faces ahead of them, from one call site (the
             // face code is emitted once)
-            const int nface = (c0 == s_begin) ? NT + FC * W : NT;
-            for (int idx = tid; idx < nface; idx += NT) {
+            const int nface = (c0 == s_begin && !ONE) ? NT + FC * W : NT;
+            for (int idx = (ONE && tp >= s_end - s_begin + FC) ? NT : tid; idx < nface; idx += NT) {
                 int l, j;
-                if (idx < NT) {
+                if (ONE || idx < NT) {
                     l = tl;
-                    j = c0 + HG - 2 + tp;
+                    j = c0 + tp + (ONE ? -FO : HG - 2);
                 } else {
                     const int e = idx - NT;
                     l = (AX == 0) ? e / FC : e % W;
@@ -574,11 +587,11 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
         }
         __syncthreads();
 
-        const int i = c0 + tp;
+        const int i = c0 + tp - (ONE ? FC : 0);
         bool ok; long long base; int lid;
         own_line(ok, base, lid);
-        if constexpr (PF) __pipeline_wait_prior(1);  // the epilogue operands; the next cell may still fly
-        if (ok && i < s_end) {
+        if constexpr (PF) __pipeline_wait_prior(ONE ? 0 : 1);  // the epilogue operands; the next cell may still fly
+        if (ok && i < s_end && (!ONE || i >= s_begin)) {
             double fnm[NV], fnp[NV];
             if constexpr (DIFF == 0) {  // node fluxes of cells i-1 and i+1 (SolvePointSolver, nl = nr = 1)
                 double pm[NV], pp[NV];
@@ -708,7 +721,7 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
                 }
             }
         }
-        __syncthreads();
+        if constexpr (!ONE) __syncthreads();
     }
 
     if (p.mode == MODE_RK) {
@@ -717,11 +730,11 @@ __device__ __forceinline__ void sweep_tile(const SweepParams &p, int block_id)
     }
 }
 
-template <int NV, int AX, int FAM, int FLUX, int S, int W, int PREC, int DIFF>
+template <int NV, int AX, int FAM, int FLUX, int S, int W, int PREC, int DIFF, bool ONE>
 __global__ void __launch_bounds__(S *W, (SweepShape<NV, AX, FAM, FLUX, S, W, PREC, DIFF>::MINB))
     sweep_kernel(const __grid_constant__ SweepParams p)
 {
-    sweep_tile<NV, AX, FAM, FLUX, S, W, PREC, DIFF>(p, (int)(p.tile0 + blockIdx.x));
+    sweep_tile<NV, AX, FAM, FLUX, S, W, PREC, DIFF, ONE>(p, (int)(p.tile0 + blockIdx.x));
     if constexpr (AX == NV - 3) {
         if (p.ctl_step) {
             __threadfence();  // this CTA's maxima before its ticket
@@ -781,11 +794,11 @@ __global__ void __launch_bounds__(S *W, (SweepShape<NV, AX, FAM, FLUX, S, W, PRE
     }
 }
 
-template <int NV, int AX, int FAM, int FLUX, int S, int W, int PREC, int DIFF>
-static cudaError_t launch_sweep_shape_p(const SweepParams &p, cudaStream_t st)
+template <int NV, int AX, int FAM, int FLUX, int S, int W, int PREC, int DIFF, bool ONE>
+static cudaError_t launch_sweep_kernel(const SweepParams &p, cudaStream_t st)
 {
     using SH = SweepShape<NV, AX, FAM, FLUX, S, W, PREC, DIFF>;
-    auto kern = sweep_kernel<NV, AX, FAM, FLUX, S, W, PREC, DIFF>;
+    auto kern = sweep_kernel<NV, AX, FAM, FLUX, S, W, PREC, DIFF, ONE>;
     // the dynamic shared-memory opt-in is per device
     static bool attr_set[64] = {};
     int dev = 0;
@@ -826,8 +839,23 @@ static cudaError_t launch_sweep_shape_p(const SweepParams &p, cudaStream_t st)
         return cudaErrorInvalidValue;
     }
     if (nblk <= 0) return cudaSuccess;
-    sweep_kernel<NV, AX, FAM, FLUX, S, W, PREC, DIFF><<<(unsigned)nblk, SH::NT, SH::SMEM_BYTES, st>>>(q);
+    kern<<<(unsigned)nblk, SH::NT, SH::SMEM_BYTES, st>>>(q);
     return cudaGetLastError();
+}
+
+template <int NV, int AX, int FAM, int S, int W, int PREC, int DIFF>
+static cudaError_t launch_sweep_shape(int flux, const SweepParams &p, cudaStream_t st)
+{
+    // The strict flavour only: there both kernels round alike, while contraction
+    // may differ between two kernels of the fast flavour, whose results must not
+    // depend on how lines are cut.
+    if constexpr (DIFF == 0 && kStrictFlavour) {
+        if (p.seg_len <= S - SweepShape<NV, AX, FAM, FLUX_ROE, S, W, PREC, DIFF>::FC)
+            return flux == FLUX_HLLC ? launch_sweep_kernel<NV, AX, FAM, FLUX_HLLC, S, W, PREC, DIFF, true>(p, st)
+                                     : launch_sweep_kernel<NV, AX, FAM, FLUX_ROE, S, W, PREC, DIFF, true>(p, st);
+    }
+    return flux == FLUX_HLLC ? launch_sweep_kernel<NV, AX, FAM, FLUX_HLLC, S, W, PREC, DIFF, false>(p, st)
+                             : launch_sweep_kernel<NV, AX, FAM, FLUX_ROE, S, W, PREC, DIFF, false>(p, st);
 }
 
 template <int NV, int AX, int FAM, int FLUX, int S, int W, int PREC>
@@ -857,77 +885,46 @@ static cudaError_t launch_batched_shape_p(const BatchSweep &b, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// FP64 or, in the fast flavour of the multi-dimensional kernels, mixed; the
-// TRAD6 difference in FP64 only.
-template <int NV, int AX, int FAM, int FLUX, int S, int W>
-static cudaError_t launch_sweep_shape(const SweepParams &p, cudaStream_t st)
-{
-    if (p.diff == DIFF_TRAD6) return p.prec == 0 ? launch_sweep_shape_p<NV, AX, FAM, FLUX, S, W, 0, 1>(p, st)
-                                                 : cudaErrorInvalidValue;
-    if (p.prec == 0) return launch_sweep_shape_p<NV, AX, FAM, FLUX, S, W, 0, 0>(p, st);
-#if defined(CFD_FAST)
-    if constexpr (NV >= 4 && FAM != FAM_RESEARCH) return launch_sweep_shape_p<NV, AX, FAM, FLUX, S, W, 1, 0>(p, st);
-#endif
-    return cudaErrorInvalidValue;
-}
-
 // Tile shapes (sweep_params.h): kXSn x kXWn along x in 3D and for 2D FP64,
 // kXS x kXW along x for the 2D mixed form; kYSm x kYWm along y and z;
-// kXS x kXW and kYS x kYW for the TRAD6 difference; k1S x k1W in 1D.
+// kXS x kXW and kYS x kYW for the TRAD6 difference (FP64 only); k1S x k1W in
+// 1D. The mixed form exists in the fast flavour of the multi-dimensional
+// kernels.
+template <int NV, int AX, int FAM>
+static cudaError_t launch_sweep_ax(int flux, const SweepParams &p, cudaStream_t st)
+{
+    if (p.diff == DIFF_TRAD6) {
+        if (p.prec != 0) return cudaErrorInvalidValue;
+        if constexpr (NV == 3) return launch_sweep_shape<NV, AX, FAM, k1S, k1W, 0, 1>(flux, p, st);
+        else if constexpr (AX == 0) return launch_sweep_shape<NV, AX, FAM, kXS, kXW, 0, 1>(flux, p, st);
+        else return launch_sweep_shape<NV, AX, FAM, kYS, kYW, 0, 1>(flux, p, st);
+    }
+    if (p.prec != 0) {
+#if defined(CFD_FAST)
+        if constexpr (NV >= 4 && FAM != FAM_RESEARCH) {
+            if constexpr (AX == 0 && NV == 4) return launch_sweep_shape<NV, AX, FAM, kXS, kXW, 1, 0>(flux, p, st);
+            else if constexpr (AX == 0) return launch_sweep_shape<NV, AX, FAM, kXSn, kXWn, 1, 0>(flux, p, st);
+            else return launch_sweep_shape<NV, AX, FAM, kYSm, kYWm, 1, 0>(flux, p, st);
+        }
+#endif
+        return cudaErrorInvalidValue;
+    }
+    if constexpr (NV == 3) return launch_sweep_shape<NV, AX, FAM, k1S, k1W, 0, 0>(flux, p, st);
+    else if constexpr (AX == 0) return launch_sweep_shape<NV, AX, FAM, kXSn, kXWn, 0, 0>(flux, p, st);
+    else return launch_sweep_shape<NV, AX, FAM, kYSm, kYWm, 0, 0>(flux, p, st);
+}
+
 template <int NV, int FAM>
 cudaError_t launch_sweep(int ax, int flux, const SweepParams &p, cudaStream_t st)
 {
-    if constexpr (NV == 3) {
-        if (ax != 0) return cudaErrorInvalidValue;
-        return flux == FLUX_HLLC ? launch_sweep_shape<3, 0, FAM, FLUX_HLLC, k1S, k1W>(p, st)
-                                 : launch_sweep_shape<3, 0, FAM, FLUX_ROE, k1S, k1W>(p, st);
-    } else {
-        if (ax == 0) {
-            // 16-cell chunks of 8 lines: faster in 3D (both forms) and for 2D FP64
-            if (p.diff != DIFF_TRAD6 && (NV == 5 || p.prec == 0))
-                return flux == FLUX_HLLC ? launch_sweep_shape<NV, 0, FAM, FLUX_HLLC, kXSn, kXWn>(p, st)
-                                         : launch_sweep_shape<NV, 0, FAM, FLUX_ROE, kXSn, kXWn>(p, st);
-            return flux == FLUX_HLLC ? launch_sweep_shape<NV, 0, FAM, FLUX_HLLC, kXS, kXW>(p, st)
-                                     : launch_sweep_shape<NV, 0, FAM, FLUX_ROE, kXS, kXW>(p, st);
-        }
-        if (ax == 1) {
-#if defined(CFD_FAST)
-            if constexpr (FAM != FAM_RESEARCH) {
-                if (p.prec == 1 && p.diff != DIFF_TRAD6)
-                    return flux == FLUX_HLLC ? launch_sweep_shape_p<NV, 1, FAM, FLUX_HLLC, kYSm, kYWm, 1, 0>(p, st)
-                                             : launch_sweep_shape_p<NV, 1, FAM, FLUX_ROE, kYSm, kYWm, 1, 0>(p, st);
-            }
-#endif
-            if constexpr ((NV == 5 && CFD_FP64_3D_YZ16) || (NV == 4 && CFD_FP64_2D_Y16)) {
-                if (p.prec == 0 && p.diff != DIFF_TRAD6)
-                    return flux == FLUX_HLLC ? launch_sweep_shape_p<NV, 1, FAM, FLUX_HLLC, kYSm, kYWm, 0, 0>(p, st)
-                                             : launch_sweep_shape_p<NV, 1, FAM, FLUX_ROE, kYSm, kYWm, 0, 0>(p, st);
-            }
-            return flux == FLUX_HLLC ? launch_sweep_shape<NV, 1, FAM, FLUX_HLLC, kYS, kYW>(p, st)
-                                     : launch_sweep_shape<NV, 1, FAM, FLUX_ROE, kYS, kYW>(p, st);
-        }
-        if constexpr (NV == 5) {
-            if (ax == 2) {
-#if defined(CFD_FAST)
-                if constexpr (FAM != FAM_RESEARCH && CFD_MIXED_Z16) {
-                    if (p.prec == 1 && p.diff != DIFF_TRAD6)
-                        return flux == FLUX_HLLC
-                                   ? launch_sweep_shape_p<NV, 2, FAM, FLUX_HLLC, kYSm, kYWm, 1, 0>(p, st)
-                                   : launch_sweep_shape_p<NV, 2, FAM, FLUX_ROE, kYSm, kYWm, 1, 0>(p, st);
-                }
-#endif
-                if constexpr (CFD_FP64_3D_YZ16) {
-                    if (p.prec == 0 && p.diff != DIFF_TRAD6)
-                        return flux == FLUX_HLLC
-                                   ? launch_sweep_shape_p<NV, 2, FAM, FLUX_HLLC, kYSm, kYWm, 0, 0>(p, st)
-                                   : launch_sweep_shape_p<NV, 2, FAM, FLUX_ROE, kYSm, kYWm, 0, 0>(p, st);
-                }
-                return flux == FLUX_HLLC ? launch_sweep_shape<NV, 2, FAM, FLUX_HLLC, kYS, kYW>(p, st)
-                                         : launch_sweep_shape<NV, 2, FAM, FLUX_ROE, kYS, kYW>(p, st);
-            }
-        }
-        return cudaErrorInvalidValue;
+    if (ax == 0) return launch_sweep_ax<NV, 0, FAM>(flux, p, st);
+    if constexpr (NV >= 4) {
+        if (ax == 1) return launch_sweep_ax<NV, 1, FAM>(flux, p, st);
     }
+    if constexpr (NV == 5) {
+        if (ax == 2) return launch_sweep_ax<NV, 2, FAM>(flux, p, st);
+    }
+    return cudaErrorInvalidValue;
 }
 
 // Persistent batched sweep (1D, 2D and 3D): the single-grid tile shapes, or for

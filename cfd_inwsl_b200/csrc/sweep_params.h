@@ -30,15 +30,6 @@ constexpr int kYS = CFD_YS, kYW = CFD_YW;  // along y and z (TRAD6, batched alte
 #define CFD_YWM 16
 #endif
 constexpr int kYSm = CFD_YSM, kYWm = CFD_YWM;  // along y and z
-#ifndef CFD_FP64_3D_YZ16
-#define CFD_FP64_3D_YZ16 1  // the FP64 3D y/z sweeps take the kYSm x kYWm shape too (0: kYS x kYW)
-#endif
-#ifndef CFD_FP64_2D_Y16
-#define CFD_FP64_2D_Y16 1  // the FP64 2D y sweep takes the kYSm x kYWm shape too (0: kYS x kYW)
-#endif
-#ifndef CFD_MIXED_Z16
-#define CFD_MIXED_Z16 1  // the mixed form's z sweep takes the kYSm x kYWm shape too (0: kYS x kYW)
-#endif
 constexpr int k1S = 128, k1W = 1;          // 1D
 
 
