@@ -21,6 +21,13 @@
 // kernel sums each cell's twelve face contributions and its two node
 // contributions (no atomics: the result is deterministic) and applies the
 // stage-adjoint combination the caller asks for.
+//
+// Bound by FP64 latency: the P buffer (24 values a face) stays in L2 at the
+// sizes adjoints run at, and 8 to 16 warps per SM have a face's dependent
+// chains to wait out. Reciprocals and roots without branches and products
+// with the eigenvectors' structural zeros left out took one product of 256^2
+// from 53.3 to 45.1 us, of 320^2 from 76.6 to 62.7 us (one B200, graph-less
+// launches back to back).
 #include "adjoint.h"
 #include "adjoint_math.h"
 
