@@ -44,6 +44,7 @@ enum : int {
     BND_SYMMETRYX = 10,
     BND_SYMMETRYY = 11,
     BND_SYMMETRYZ = 12,
+    BND_PERIODIC_WRAP = 100,  // in SweepParams::bc_type only; the tables hold PERIODIC1D wired as a wrap
     BND_HALO = 101,      // ghost cells from a neighbour's rows (slab decomposition): i0 = line, offset = side
 };
 
@@ -143,6 +144,7 @@ struct SweepParams {
     unsigned *err;      // ErrBits
     const BcLine *bc_lo;  // per line (index a + n[T0] * b), low end
     const BcLine *bc_hi;  // per line, high end
+    int bc_type[2];       // FP64 sweeps without tables (both null): the type of every low / high line end
     const double *bc_vals; // static ghost prim values [slot][ghosts per side][NV]
     double t;           // stage time (ignored when ctl is set)
     const StepCtl *ctl; // device-resident step control (null: use rkBdt/t)
