@@ -50,13 +50,13 @@ constexpr double kRcpGm1 = 1.0 / kGm1;          // RN(1 / (gamma - 1))
 // within one ulp of a/b and y = RN(1/b), the residual r = a - b q is exact in
 // an FMA and RN(q + r y) = RN(a/b). q0 = RN(a y) can lie slightly more than
 // one ulp away, so a first correction brings it within a small fraction of an
-// ulp and a second applies the theorem: five FP64 operations against about
-// thirteen FP64 issue slots for a division on B200 (measured). Dividends that
+// ulp and a second applies the theorem. Dividends that
 // are tiny (below 2^-960, where the residual could be subnormal), huge or not
 // finite take the IEEE division itself; zeros keep their sign through the
-// sign of RN(a y). Quotients formed together share one test and one branch
-// (divs_rn). The denominators here are densities, sound speeds, enthalpies
+// sign of RN(a y). The denominators here are densities, sound speeds, enthalpies
 // and spacings, normal numbers far from the ends of the exponent range.
+// This form serves the kernels beside the sweeps and the sweeps' out-of-line
+// path; the sweeps themselves divide by OpsSpec below.
 // ---------------------------------------------------------------------------
 CFD_HD double rcp_rn(double b)
 {
@@ -114,7 +114,7 @@ template <int N>
 struct DivN {
     double v[N];
 };
-// A group's IEEE divisions, out of line (one call site per group)
+// A group's IEEE divisions, out of line
 template <int N>
 static __device__ __noinline__ DivN<N> divs_ieee(DivN<N> a, DivN<N> b)
 {
@@ -124,35 +124,6 @@ static __device__ __noinline__ DivN<N> divs_ieee(DivN<N> a, DivN<N> b)
     return q;
 }
 #endif
-
-// q[i] = RN(a[i] / b[i]), y[i] = RN(1/b[i]), for N quotients formed together:
-// one branch to the IEEE division for the group instead of one per quotient.
-template <int N>
-CFD_HD void divs_rn(const double *a, const double *b, const double *y, double *q)
-{
-#if defined(__CUDA_ARCH__)
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        q[i] = mk_div(a[i], b[i], y[i]);
-        ok = ok & mk_ok(a[i]);
-    }
-    if (!ok) {
-        DivN<N> A, B;
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            A.v[i] = a[i];
-            B.v[i] = b[i];
-        }
-        const DivN<N> Q = divs_ieee<N>(A, B);
-#pragma unroll
-        for (int i = 0; i < N; i++) q[i] = Q.v[i];
-    }
-#else
-    (void)y;
-    for (int i = 0; i < N; i++) q[i] = a[i] / b[i];
-#endif
-}
 
 // ---------------------------------------------------------------------------
 // Arithmetic policies of the pointwise functions below.

@@ -4,9 +4,9 @@
 // library do it: code running inside another framework's memory pool or
 // arena, or a host program that has reserved all device memory up front. They
 // pass device buffers for the input state and the output RHS; the only scratch
-// this entry point needs, the ghost-cell wiring of every line end, lives in a
-// fixed file-scope device array that every GPU loading the library holds until
-// the process exits.
+// this entry point needs, the ghost-cell wiring of every line end of a grid
+// with a DoubleMachUp side, lives in a fixed file-scope device array that every
+// GPU loading the library holds until the process exits.
 //
 // Compiled with --fmad=false like api.cu.
 #include "cfdgpu.h"

@@ -211,9 +211,10 @@ int cfd_fp64_peak_probe(long long iters, void *stream, double *flops);
 /* Self-check of the strict flavour's correctly rounded division by a shared
  * reciprocal (Markstein's correction) against the device's IEEE division on n
  * seeded operand pairs (random, next to rounding midpoints, physical ranges,
- * signed zeros, tiny and huge dividends), each also in the grouped form
- * (three dividends over one divisor of either sign); *mismatches counts
- * quotients or reciprocals whose bits differ. No counterpart in the reference: it
+ * signed zeros, tiny and huge dividends), and of the sweeps' branch-free
+ * quotients, reciprocals and square roots where they accept the operands
+ * (significands next to the ends of a binade and squares next to rounding
+ * boundaries among them); *mismatches counts results whose bits differ. No counterpart in the reference: it
  * backs the strict flavour's bit-for-bit parity. */
 int cfd_check_division(long long n, unsigned long long seed, unsigned long long *mismatches);
 
@@ -241,8 +242,9 @@ int cfd_eval_face(int dim, int ax, int inter_method, int precision, const double
  * stream) without synchronising. It calls no cudaMalloc/cudaFree and no
  * allocating library routine.
  *
- * Its only scratch, the ghost wiring of every line end, lives in a file-scope
- * device array of CFD_NOALLOC_MAX_LINE_ENDS entries (768 KiB) that each GPU
+ * Its only scratch, the ghost wiring of every line end of a grid with a
+ * DoubleMachUp side (others need none), lives in a file-scope device array of
+ * CFD_NOALLOC_MAX_LINE_ENDS entries (768 KiB) that each GPU
  * loading the library holds until the process exits. Grids with more line
  * ends than that (sum over directions of 2 * ncell / n[d]; 2D grids up to
  * 4096 x 4096 fit) are rejected with CFD_ERR_CONFIG and a message on stderr.
@@ -253,8 +255,9 @@ int cfd_eval_face(int dim, int ax, int inter_method, int precision, const double
  * context, this entry point must not be called on that device again in the
  * same process. cfg->bc takes the same types as in cfd_create. A CUDA error
  * already pending on the calling thread is left in place and the call
- * returns CFD_ERR_CUDA without queueing anything. Every call rewrites the part of the array it uses, and all
- * calls share it: calls that overlap on the GPU (different streams, or other
+ * returns CFD_ERR_CUDA without queueing anything. Every call on a grid with a
+ * DoubleMachUp side rewrites the part of the array it uses, and all such
+ * calls share it: those that overlap on the GPU (different streams, or other
  * threads) race on the array and must be serialised by the caller. */
 #define CFD_NOALLOC_MAX_LINE_ENDS 16384
 int cfd_rhs_noalloc(const cfd_config *cfg, const double *cons_soa, double *rhs_soa, double t, void *stream);
