@@ -302,16 +302,19 @@ struct SweepShape {
     static constexpr int SMEM_FLOATS = PREC ? 2 * NV * W * LSP : 0;
     // Resident CTAs per SM the launch bounds ask for: 512 threads per SM in
     // 2D/3D (two CTAs of 256 threads or four of 128), 128 registers a thread;
-    // or three 128-thread CTAs (168 registers, fewer spills), which measured
-    // faster for the FP64 y sweep (2D), every FP64 3D sweep (the x sweep
-    // spilled 880 / 576 bytes per thread at 128 registers in the strict /
-    // fast flavour: 3.35 -> 3.23 and 1.90 -> 1.78 ms per 256^3 launch at
-    // three CTAs), the FP64 TENO-Z x sweep and the 3D mixed TENO-Z sweeps.
-    static constexpr bool THREE = ((FAM == FAM_TENOZ) && (PREC == 0 ? AX == 0 : NV == 5)) ||
-                                  (PREC == 0 && NV == 5) || (PREC == 0 && NV == 4 && AX == 1);
-    // The strict flavour's 3D z sweep (the stage-closing one) measured 7%
-    // faster at two CTAs per SM (255 registers) than at three.
-    static constexpr bool TWO = kStrictFlavour && PREC == 0 && NV == 5 && AX == 2;
+    // or three 128-thread CTAs (168 registers, fewer spills). Timed again on
+    // the branch-free arithmetic, four against three: 2D WCNS5 x 256 against
+    // 261 us fast and 379 against 400 strict, y 334 against 287 fast; 2D TENO
+    // strict x 356 against 346, y 468 against 378 (2048^2); 3D WCNS5 fast x 166
+    // against 173, y 176 against 171, z 210 against 197 (128^3), strict x 260
+    // against 266, y 275 against 276, z 303 against 308 at two (255
+    // registers). So four for WCNS5 along x and for the strict 3D WCNS5
+    // sweeps, and three, as before, for 2D y, 3D and the FP64 TENO-Z x sweep,
+    // and the 3D mixed TENO-Z sweeps; two for the other families' strict z.
+    static constexpr bool FOUR = PREC == 0 && NV == 5 && FAM == FAM_WCNS5 && (AX == 0 || kStrictFlavour);
+    static constexpr bool THREE = !FOUR && (((FAM == FAM_TENOZ) && (PREC == 0 ? AX == 0 : NV == 5)) ||
+                                            (PREC == 0 && NV == 5) || (PREC == 0 && NV == 4 && AX == 1));
+    static constexpr bool TWO = !FOUR && kStrictFlavour && PREC == 0 && NV == 5 && AX == 2;
     static constexpr int MINB128 = TWO ? 2 : THREE ? 3 : CFD_SWEEP_MINB128;
     static constexpr int MINB = (NT <= 256) ? (NV >= 4 ? (NT == 128 ? MINB128 : CFD_SWEEP_MINB * (256 / NT))
                                                        : CFD_SWEEP_MINB)
