@@ -27,6 +27,7 @@ using cfd::SweepParams;
 
 namespace cfd {
 int default_seg_len_for(const cfd_config *cfg, int d);
+int seg_len_for(const cfd_config *cfg, int d, int n, long long parts);
 bool config_bc_ok(const cfd_config *cfg, const char **why);
 }
 
@@ -1146,10 +1147,8 @@ int cfd_step_host(cfd_handle *h, double cfl, double output_dt, const double *in_
     const int L = h->dim - 1;
     const long long nL = h->cfg.n[L];
     const long long plane = h->ncell / nL;  // cells per index of the last dimension
-    const long long seg = h->seg_len[L];
-    const long long nseg = (nL + seg - 1) / seg;
     int rc;
-    if (h->dim < 2 || nL < 64 || nseg < 2) {
+    if (h->dim < 2 || nL < 64 || nL <= h->seg_len[L]) {
         // too small to overlap: the three calls in turn
         if ((rc = cfd_upload_cons(h, in_aos))) return rc;
         int ns = 0;
@@ -1197,6 +1196,16 @@ int cfd_step_host(cfd_handle *h, double cfl, double output_dt, const double *in_
     // rounding of the epilogue it replaces.
     const long long lines_up = ((nL + kHostChunks - 1) / kHostChunks + 31) / 32 * 32;
     const int nup = (int)((nL + lines_up - 1) / lines_up);
+    // A chunk's launch has an eighth of the grid's CTAs: its segments are cut
+    // for that (520 x 869 fast: 0.95 -> 0.81 ms a step), unless the
+    // configuration says otherwise.
+    auto chunk_seg = [&](int d) -> int {
+        if (h->cfg.seg_len[d] > 0) return h->seg_len[d];
+        return std::min(h->seg_len[d], d == L ? cfd::seg_len_for(&h->cfg, d, (int)std::min(nL, lines_up), 1)
+                                              : cfd::seg_len_for(&h->cfg, d, h->cfg.n[d], nup));
+    };
+    const long long seg = chunk_seg(L);
+    const long long nseg = (nL + seg - 1) / seg;
     const long long tail0 = (long long)(nup - 1) * lines_up;  // first row of the last chunk
     const bool early_last = !h->line_bc_set[L];
     const long long halo = 5;  // ghost cells each side of a segment (4 with MND6, 5 with TRAD6)
@@ -1205,6 +1214,7 @@ int cfd_step_host(cfd_handle *h, double cfl, double output_dt, const double *in_
         if (s1 <= s0) return CFD_OK;
         SweepParams p = stage_params(h, L, 1, U0, U0, U1, 1.0, 0.0, 0.0, 0.0, false, h->ctl);
         p.mode = cfd::MODE_WRITE;  // the RHS only; rk_combine applies the stage
+        p.seg_len = (int)seg;
         p.part_lo = (int)(s0 * seg);
         p.part_hi = (int)std::min(nL, s1 * seg);
         p.seg_outer = 1;
@@ -1220,6 +1230,7 @@ int cfd_step_host(cfd_handle *h, double cfl, double output_dt, const double *in_
         if ((rc = launch_aos_to_soa(h, h->stage, U0, c0, c1)) || (rc = launch_wave_speed_range(h, c0, c1))) return rc;
         for (int d = 0; d < L; d++) {
             SweepParams p = stage_params(h, d, 1, U0, U0, U1, 1.0, 0.0, 0.0, 0.0, false, h->ctl);
+            p.seg_len = chunk_seg(d);
             p.part_lo = (int)r0;
             p.part_hi = (int)r1;
             if ((rc = sweep(h, d, p))) return rc;
@@ -1255,6 +1266,7 @@ int cfd_step_host(cfd_handle *h, double cfl, double output_dt, const double *in_
     for (long long s0 = 0; s0 < nseg; s0 += segs_dn, k++) {
         const long long r0 = s0 * seg, r1 = std::min(nL, (s0 + segs_dn) * seg), c0 = r0 * plane, c1 = r1 * plane;
         SweepParams p = stage_params(h, L, 3, U2, U0, U1, 1.0 / 3.0, 0.0, 2.0 / 3.0, 0.0, true, h->ctl);
+        p.seg_len = (int)seg;
         p.part_lo = (int)r0;
         p.part_hi = (int)r1;
         p.seg_outer = 1;
@@ -1481,9 +1493,12 @@ namespace cfd {
 // Default cells per CTA segment along direction d for the tile shapes that
 // launch_sweep picks for this configuration. Shared with the allocation-free
 // entry point (noalloc.cu).
-int default_seg_len_for(const cfd_config *cfg, int d)
+int default_seg_len_for(const cfd_config *cfg, int d) { return seg_len_for(cfg, d, cfg->n[d], 1); }
+
+// The same for a launch that covers n cells along d of one in `parts` of the
+// lines (the chunks of cfd_step_host).
+int seg_len_for(const cfd_config *cfg, int d, int n, long long parts)
 {
-    const int n = cfg->n[d];
     // the shapes of launch_sweep_ax
     const bool trad6 = cfg->diff_method == CFD_DIFF_TRAD6;
     const bool wide_x = trad6 || (cfg->dim == 2 && cfg->precision == CFD_PREC_MIXED);
@@ -1492,6 +1507,7 @@ int default_seg_len_for(const cfd_config *cfg, int d)
     int t0, t1;
     transverse_axes(d, t0, t1);
     long long blocks_per_seg = (long long)((cfg->n[t0] + W - 1) / W) * cfg->n[t1];
+    blocks_per_seg = (blocks_per_seg + parts - 1) / parts;
     // about 1,800 CTAs (3 to 6 waves at 2 to 4 resident per SM); the mixed
     // form's x sweep measured fastest with half as many, longer segments
     const bool mixed_x = d == 0 && cfg->dim > 1 && cfg->precision == CFD_PREC_MIXED;
