@@ -371,7 +371,9 @@ struct cfd_handle {
     size_t d_bcvals_cap = 0;
     bool bc_dirty = true;
     int seg_len[3] = {1, 1, 1};
-    bool ws_valid = false;       // red[1..3] hold the wave speeds of the current state
+    // red[1..3] hold the wave speeds of the current state; cleared before a call
+    // consumes them, so that a call that fails on the way leaves none behind
+    bool ws_valid = false;
     double dm_u = 0.0, dm_v = 0.0;
     std::string msg;
     cudaStream_t own_stream = nullptr;   // created by cfd_create
@@ -1064,6 +1066,7 @@ int cfd_rk3_step(cfd_handle *h, double dt, double t, double *rho_linf)
     double t1 = t, t2 = t + dt, t3 = t2 - dt / 2;
     if ((rc = rk_stage(h, 1, U0, U0, U1, 1.0, dt, 0.0, t1, false))) return rc;
     if ((rc = rk_stage(h, 2, U1, U0, U2, 0.75, 0.25 * dt, 0.25, t2, false))) return rc;
+    h->ws_valid = false;
     CFD_CUDA(h, cudaMemsetAsync(h->red, 0, 4 * sizeof(unsigned long long), h->stream));
     if ((rc = rk_stage(h, 3, U2, U0, U1, 1.0 / 3.0, 2.0 / 3.0 * dt, 2.0 / 3.0, t3, true))) return rc;
     h->cur = (h->cur + 1) % 3;
@@ -1098,6 +1101,7 @@ int cfd_run(cfd_handle *h, double cfl, int end_step, double output_dt, int max_s
     c->maxSteps = max_steps;
     CFD_CUDA(h, cudaMemcpyAsync(h->ctl, c, sizeof(*c), cudaMemcpyHostToDevice, h->stream));
     CFD_CUDA(h, cudaMemsetAsync(h->err, 0, 2 * sizeof(unsigned), h->stream));
+    h->ws_valid = false;  // consumed by step_begin
     step_begin_kernel<<<1, 1, 0, h->stream>>>(h->ctl, h->red, h->dim, h->d_dts);
     CFD_CUDA(h, cudaGetLastError());
     h->launches++;
@@ -1125,7 +1129,6 @@ int cfd_run(cfd_handle *h, double cfl, int end_step, double output_dt, int max_s
         if (c->done || launched >= max_steps) break;
         if (quota < (1 << 20)) quota *= 2;
     }
-    // a step that met the loop test before `done` was set still has to finish
     int k = c->k;
     *nsteps = k;
     *t = c->t;
@@ -1177,6 +1180,7 @@ int cfd_step_host(cfd_handle *h, double cfl, double output_dt, const double *in_
     c->tst[1] = *t;
     CFD_CUDA(h, cudaMemcpyAsync(h->ctl, c, sizeof(*c), cudaMemcpyHostToDevice, st));
     CFD_CUDA(h, cudaMemsetAsync(h->err, 0, sizeof(unsigned), st));
+    h->ws_valid = false;
     CFD_CUDA(h, cudaMemsetAsync(h->red, 0, 4 * sizeof(unsigned long long), st));
     // the copies start after the work queued so far on the handle's stream
     CFD_CUDA(h, cudaEventRecord(h->host_ev[1][0], st));
@@ -2502,6 +2506,7 @@ int cfd_rk3_stage(cfd_handle *h, int stage, double dt, double t)
         return rk_stage(h, 1, U0, U0, U1, 1.0, dt, 0.0, t, false);
     }
     if (stage == 2) return rk_stage(h, 2, U1, U0, U2, 0.75, 0.25 * dt, 0.25, t2, false);
+    h->ws_valid = false;
     CFD_CUDA(h, cudaMemsetAsync(h->red, 0, 4 * sizeof(unsigned long long), h->stream));
     if ((rc = rk_stage(h, 3, U2, U0, U1, 1.0 / 3.0, 2.0 / 3.0 * dt, 2.0 / 3.0, t3, true))) return rc;
     h->cur = (h->cur + 1) % 3;

@@ -70,8 +70,9 @@ enum SweepMode : int { MODE_WRITE = 0, MODE_RK = 2 };
 enum ErrBits : unsigned { ERR_NONFINITE = 1u, ERR_NEGATIVE = 2u, ERR_TIMEOUT = 4u };
 
 // Device-resident state of the time loop of BlockSolver::stepsLoopCFL
-// (blockSolver.cpp:170-235), advanced by single-thread control kernels so that
-// whole steps can be captured in CUDA graphs without host round trips.
+// (blockSolver.cpp:170-235), advanced by one thread (a control kernel, or the
+// last CTA of a step's last sweep) so that whole steps can be captured in CUDA
+// graphs without host round trips.
 struct StepCtl {
     double t, outputT, outputDt, cfl, dt;
     double bdt[4];   // per stage: dt, 0.25*dt, (2/3)*dt (index = stage)
