@@ -26,7 +26,7 @@
 // sizes adjoints run at, and 8 to 16 warps per SM have a face's dependent
 // chains to wait out. Reciprocals and roots without branches and products
 // with the eigenvectors' structural zeros left out took one product of 256^2
-// from 53.3 to 45.1 us, of 320^2 from 76.6 to 62.7 us (one B200, graph-less
+// from 53.3 to 45.1 us, of 320^2 from 76.6 to 63.0 us (one B200, graph-less
 // launches back to back).
 #include "adjoint.h"
 #include "adjoint_math.h"

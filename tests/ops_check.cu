@@ -1,0 +1,75 @@
+// Device evaluation of single operations of the library's arithmetic headers
+// for tests/test_gpu_ops.py: operand rows in, result rows out, beside the
+// compiler's own operations where a comparison needs them.
+#include "adjoint_math.h"
+
+#include <cuda_runtime.h>
+
+namespace {
+
+struct Arcp {  // 1/b and the compiler's
+    static constexpr int in = 1, out = 2;
+    static __device__ void f(const double *x, double *r)
+    {
+        r[0] = cfd::adj::arcp(x[0]);
+        r[1] = 1.0 / x[0];
+    }
+};
+struct Asqrt {
+    static constexpr int in = 1, out = 2;
+    static __device__ void f(const double *x, double *r)
+    {
+        r[0] = cfd::adj::asqrt(x[0]);
+        r[1] = sqrt(x[0]);
+    }
+};
+struct Wcns5Adj {  // five stencil values and the result's adjoint
+    static constexpr int in = 6, out = 5;
+    static __device__ void f(const double *x, double *r)
+    {
+        for (int i = 0; i < 5; i++) r[i] = 0.0;
+        cfd::adj::wcns5_adj(x, x[5], r);
+    }
+};
+struct FaceVjp {  // six cells' cons and the adjoint of the flux, along x
+    static constexpr int in = 28, out = 24;
+    static __device__ void f(const double *x, double *r)
+    {
+        double U[6][4], Ub[6][4] = {};
+        for (int j = 0; j < 24; j++) U[j / 4][j % 4] = x[j];
+        cfd::adj::face_vjp<0>(U, x + 24, Ub);
+        for (int j = 0; j < 24; j++) r[j] = Ub[j / 4][j % 4];
+    }
+};
+
+template <class OP>
+__global__ void each(const double *x, double *r, long n)
+{
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        OP::f(x + i * OP::in, r + i * OP::out);
+}
+
+template <class OP>
+int run(const double *x, double *r, long n)
+{
+    double *dx = nullptr, *dr = nullptr;
+    cudaError_t e = cudaMalloc(&dx, sizeof(double) * OP::in * n);
+    if (e == cudaSuccess) e = cudaMalloc(&dr, sizeof(double) * OP::out * n);
+    if (e == cudaSuccess) e = cudaMemcpy(dx, x, sizeof(double) * OP::in * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        each<OP><<<148 * 4, 128>>>(dx, dr, n);
+        e = cudaMemcpy(r, dr, sizeof(double) * OP::out * n, cudaMemcpyDeviceToHost);
+    }
+    cudaFree(dx);
+    cudaFree(dr);
+    return (int)e;
+}
+
+} // namespace
+
+extern "C" {
+int ops_arcp(const double *x, double *r, long n) { return run<Arcp>(x, r, n); }
+int ops_asqrt(const double *x, double *r, long n) { return run<Asqrt>(x, r, n); }
+int ops_wcns5_adj(const double *x, double *r, long n) { return run<Wcns5Adj>(x, r, n); }
+int ops_face_vjp(const double *x, double *r, long n) { return run<FaceVjp>(x, r, n); }
+}

@@ -1,0 +1,134 @@
+"""The arithmetic headers' own reciprocals, quotients and roots on the device,
+operation by operation, against the compiler's (tests/ops_check.cu, built here
+with the library's flags)."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
+INF, NAN = np.inf, np.nan
+
+
+@pytest.fixture(scope="module")
+def ops(tmp_path_factory):
+    """ops(flavour, name, rows, nout): result rows of one operation."""
+    from tests.conftest import gpu_available
+    if not gpu_available():
+        pytest.skip("no CUDA device")
+    from cfd_inwsl_b200 import build_ext
+    try:
+        nvcc = build_ext.nvcc_path()
+    except RuntimeError:
+        pytest.skip("no nvcc")
+    libs = {}
+
+    def call(flavour, name, rows, nout):
+        if flavour not in libs:
+            out = tmp_path_factory.mktemp("ops") / f"ops_{flavour}.so"
+            flags = ["--fmad=false"] if flavour == "strict" else ["--fmad=true", "-DCFD_FAST"]
+            subprocess.run([nvcc] + build_ext.common_flags() + flags + ["-shared", str(ROOT / "tests" / "ops_check.cu"),
+                                                                        "-o", str(out)], check=True)
+            libs[flavour] = C.CDLL(str(out))
+        x = np.ascontiguousarray(rows, dtype=np.float64)
+        r = np.empty((len(x), nout))
+        f = getattr(libs[flavour], "ops_" + name)
+        f.argtypes = [C.c_void_p, C.c_void_p, C.c_long]
+        assert f(x.ctypes.data, r.ctypes.data, len(x)) == 0
+        return r
+
+    return call
+
+
+def normals(rng, n, lo, hi):
+    """Positive numbers with exponents lo .. hi - 1, significands random and
+    next to the ends of a binade."""
+    m = 1 + rng.random(n)
+    k = rng.random(n)
+    ulps = rng.integers(0, 16, n)
+    m = np.where(k < 0.2, 2 - (1 + ulps) * 2.0**-52, m)
+    m = np.where(k > 0.8, 1 + ulps * 2.0**-52, m)
+    return np.ldexp(m, rng.integers(lo, hi, n))
+
+
+def test_adjoint_reciprocal_and_root(ops):
+    """Within an ulp of the compiler's for normal operands: a cubic step from a
+    seed off by less than 2^-18 leaves 2^-54, and one rounding half an ulp."""
+    rng = np.random.default_rng(1)
+    b = normals(rng, 1 << 20, -1022, 1022) * rng.choice([-1.0, 1.0], 1 << 20)
+    got, want = ops("fast", "arcp", b[:, None], 2).T
+    assert (np.abs(got - want) <= np.spacing(np.abs(want))).all()
+    x = normals(rng, 1 << 20, -900, 1022)
+    got, want = ops("fast", "asqrt", x[:, None], 2).T
+    assert (np.abs(got - want) <= np.spacing(want)).all()
+
+
+def test_adjoint_of_an_overflowed_measure(ops):
+    """A stencil whose outer value overflows a smoothness measure: its weight is
+    0, and the gradient is that of the candidates left, finite and with a sum
+    of 1 (each candidate reproduces a constant)."""
+    rng = np.random.default_rng(2)
+    rows = []
+    for big in (1e155, -1e160, 1e200):
+        for at in (0, 4):
+            q = rng.normal(size=5) * 1e-3
+            q[at] = big
+            rows.append([*q, 1.0])
+    g = ops("fast", "wcns5_adj", rows, 5)
+    assert np.isfinite(g).all()
+    # the measures' own derivatives sum to rounding: beta does not see a constant
+    np.testing.assert_allclose(g.sum(1), 1.0, rtol=0, atol=1e-9)
+
+
+def left_density(U):
+    """Density of the left face state of six cells' cons along x (WCNS5)."""
+    def prim(c):
+        u, v = c[1] / c[0], c[2] / c[0]
+        p = 0.4 * (c[3] - 0.5 * c[0] * (u * u + v * v))
+        return np.sqrt(c[0]), u, v, 0.5 * (u * u + v * v) + 3.5 * p / c[0]
+    (s1, u1, v1, H1), (s2, u2, v2, H2) = prim(U[2]), prim(U[3])
+    u, v, H = ((s1 * a + s2 * b) / (s1 + s2) for a, b in ((u1, u2), (v1, v2), (H1, H2)))
+    ek = 0.5 * (u * u + v * v)
+    h = H - ek
+    c = np.sqrt(0.4 * h)
+    rows = [[h - ek, u, v, -1.0], [0.5 * (u / c + ek / h), 0.5 * (-1 / c - u / h), -0.5 * v / h, 0.5 / h],
+            [0.5 * (-u / c + ek / h), 0.5 * (1 / c - u / h), -0.5 * v / h, 0.5 / h]]
+    Q = []
+    for L in rows:
+        q = U[:5] @ np.array(L)
+        s = [1e-6 + (q[0] - 2 * q[1] + q[2])**2 + 0.25 * (q[0] - 4 * q[1] + 3 * q[2])**2,
+             1e-6 + (q[1] - 2 * q[2] + q[3])**2 + 0.25 * (q[1] - q[3])**2,
+             1e-6 + (q[2] - 2 * q[3] + q[4])**2 + 0.25 * (3 * q[2] - 4 * q[3] + q[4])**2]
+        w = np.array([1 / 16, 5 / 8, 5 / 16]) / np.square(s)
+        cand = [0.375 * q[0] - 1.25 * q[1] + 1.875 * q[2], -0.125 * q[1] + 0.75 * q[2] + 0.375 * q[3],
+                0.375 * q[2] + 0.75 * q[3] - 0.125 * q[4]]
+        Q.append(w @ cand / w.sum())
+    return Q[0] / h + Q[1] + Q[2]
+
+
+def test_face_density_that_cancels(ops):
+    """Faces whose left density lies within a few roundings of zero, zero
+    itself among them: its pressure is then -inf, which takes the positivity
+    fallback, so every gradient is finite. Small amplitudes keep the weights
+    linear, so that a high second cell pulls the interpolated density down to
+    zero."""
+    rng = np.random.default_rng(3)
+    rows = []
+    for _ in range(200):
+        u, v = rng.uniform(0.2, 0.6, (2, 6))
+
+        def cells(t):
+            rho = 1e-3 * np.array([1.0, t, 0.1, 0.1, 1.0, 1.0])
+            return np.stack([rho, rho * u, rho * v, 1e-3 / 0.4 + 0.5 * rho * (u * u + v * v)], -1)
+
+        lo, hi = 0.1, 1.0
+        assert left_density(cells(lo)) > 0 > left_density(cells(hi))
+        for _ in range(60):
+            mid = 0.5 * (lo + hi)
+            lo, hi = (mid, hi) if left_density(cells(mid)) > 0 else (lo, mid)
+        for k in range(-40, 41):
+            rows.append([*cells(lo + k * np.spacing(lo)).ravel(), *rng.normal(size=4)])
+    assert np.isfinite(ops("fast", "face_vjp", rows, 24)).all()
