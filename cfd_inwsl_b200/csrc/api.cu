@@ -1670,9 +1670,10 @@ struct cfd_batch {
     // work-list order: cases by decreasing cell count, so that the persistent
     // CTAs take the longest tiles first and the tail holds the short ones
     std::vector<int> order;
-    // tiling per direction, chosen by cfd_batch_autotune: tile shape (0 the
-    // single-grid shape, 1 the alternative), segments per line (at first
-    // batch_default_split), one persistent CTA per SM instead of as many as fit
+    // tiling per direction, chosen by cfd_batch_autotune: tile shape
+    // (BatchSweep::shape; at first the single grid's), segments per line (at
+    // first batch_default_split), one persistent CTA per SM instead of as many
+    // as fit
     int shape[3] = {0, 0, 0}, split[3] = {1, 1, 1}, one_cta[3] = {0, 0, 0};
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
@@ -1724,16 +1725,18 @@ SweepParams batch_params(cfd_batch *b, int c, int slot, int stage, int d)
 int batch_chunk(const cfd_batch *b, int d)
 {
     if (b->nv == 3) return cfd::k1S;
-    if (d == 0) return (b->shape[0] || (b->nv == 4 && b->prec)) ? cfd::kXS : cfd::kXSn;
-    return b->shape[d] ? cfd::kYS : cfd::kYSm;
+    const bool single = b->shape[d] || b->prec;  // the single grid's shape
+    if (d == 0) return (!single || (b->nv == 4 && b->prec)) ? cfd::kXS : cfd::kXSn;
+    return single ? cfd::kYSm : cfd::kYS;
 }
 
 // Lines per CTA of the same sweep.
 int batch_lines(const cfd_batch *b, int d)
 {
     if (b->nv == 3) return cfd::k1W;
-    if (d == 0) return (b->shape[0] || (b->nv == 4 && b->prec)) ? cfd::kXW : cfd::kXWn;
-    return b->shape[d] ? cfd::kYW : cfd::kYWm;
+    const bool single = b->shape[d] || b->prec;
+    if (d == 0) return (!single || (b->nv == 4 && b->prec)) ? cfd::kXW : cfd::kXWn;
+    return single ? cfd::kYWm : cfd::kYW;
 }
 
 // Segments per line the batch starts with along d: the least of all CTAs'
@@ -1888,7 +1891,10 @@ int cfd_batch_create(const cfd_config *cfgs, int ncases, cfd_batch **out)
     for (int c = 0; c < ncases; c++) b->order[c] = c;
     std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) { return b->h[x]->ncell > b->h[y]->ncell; });
     // the config's seg_len of each case is replaced by the batch's tiling
-    for (int d = 0; d < b->dim; d++) b->split[d] = batch_default_split(b, d);
+    for (int d = 0; d < b->dim; d++) {
+        b->shape[d] = (b->nv >= 4 && b->prec == 0) ? 1 : 0;
+        b->split[d] = batch_default_split(b, d);
+    }
     if ((e = cudaMalloc(&b->d_tile_start, sizeof(long long) * b->dim * (ncases + 1))) != cudaSuccess) return bail(e);
     int rc = batch_layout(b);
     if (rc) {
@@ -2030,7 +2036,7 @@ int cfd_batch_set_tiling(cfd_batch *b, int idim, int shape, int segments, int on
         one_cta > 1)
         return bfail(b, CFD_ERR_CONFIG, "bad tiling");
     if (shape == 1 && !(b->nv >= 4 && b->prec == 0))
-        return bfail(b, CFD_ERR_UNSUPPORTED, "the alternative tile shape is 2D/3D FP64 only");
+        return bfail(b, CFD_ERR_UNSUPPORTED, "tile shape 1 is 2D/3D FP64 only");
     b->shape[d] = shape;
     b->split[d] = segments;
     b->one_cta[d] = one_cta;
@@ -2049,7 +2055,7 @@ int cfd_batch_autotune(cfd_batch *b, int *choice, double *ms)
     std::memset(b->ctl_host, 0, sizeof(cfd::StepCtl) * b->ncases);
     CFD_BCUDA(b, cudaMemcpyAsync(b->ctl, b->ctl_host, sizeof(cfd::StepCtl) * b->ncases, cudaMemcpyHostToDevice,
                                  b->stream));
-    const bool alt = b->nv >= 4 && b->prec == 0;  // the alternative shapes: 2D/3D FP64
+    const bool alt = b->nv >= 4 && b->prec == 0;  // 2D/3D FP64 has two shapes
     cudaEvent_t e0, e1;
     CFD_BCUDA(b, cudaEventCreate(&e0));
     CFD_BCUDA(b, cudaEventCreate(&e1));

@@ -960,8 +960,8 @@ cudaError_t launch_sweep(int ax, int flux, const SweepParams &p, cudaStream_t st
     return cudaErrorInvalidValue;
 }
 
-// Persistent batched sweep (1D, 2D and 3D): the single-grid tile shapes, or for
-// 2D/3D FP64 with b.shape = 1 the alternatives.
+// Persistent batched sweep (1D, 2D and 3D): the single-grid tile shapes, which
+// 2D/3D FP64 has as b.shape = 1 beside the longer tiles of b.shape = 0.
 template <int NV, int AX, int FAM, int S, int W, int PREC>
 static cudaError_t launch_batched_flux(int flux, const BatchSweep &b, cudaStream_t st)
 {
@@ -984,11 +984,11 @@ static cudaError_t launch_batched_ax(int flux, const BatchSweep &b, cudaStream_t
         return cudaErrorInvalidValue;
     }
     if constexpr (AX == 0)
-        return b.shape ? launch_batched_flux<NV, AX, FAM, kXS, kXW, 0>(flux, b, st)
-                       : launch_batched_flux<NV, AX, FAM, kXSn, kXWn, 0>(flux, b, st);
+        return b.shape ? launch_batched_flux<NV, AX, FAM, kXSn, kXWn, 0>(flux, b, st)
+                       : launch_batched_flux<NV, AX, FAM, kXS, kXW, 0>(flux, b, st);
     else
-        return b.shape ? launch_batched_flux<NV, AX, FAM, kYS, kYW, 0>(flux, b, st)
-                       : launch_batched_flux<NV, AX, FAM, kYSm, kYWm, 0>(flux, b, st);
+        return b.shape ? launch_batched_flux<NV, AX, FAM, kYSm, kYWm, 0>(flux, b, st)
+                       : launch_batched_flux<NV, AX, FAM, kYS, kYW, 0>(flux, b, st);
 }
 
 template <int NV, int FAM>

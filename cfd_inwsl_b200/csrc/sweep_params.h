@@ -185,7 +185,7 @@ struct BatchSweep {
     long long total_tiles;
     int num_sms;
     int prec;
-    int shape;      // 0: the single-grid tile shapes, 1: the alternative (kXS x kXW / kYS x kYW; 2D/3D FP64 only)
+    int shape;      // 2D/3D FP64: 1 the single-grid tile shapes, 0 kXS x kXW / kYS x kYW; others 0, their only one
     int one_cta;    // 1: one persistent CTA per SM, 0: as many as fit
 };
 

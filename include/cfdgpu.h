@@ -293,8 +293,9 @@ int cfd_batch_run(cfd_batch *b, double cfl, int end_step, const double *output_d
 /* Autotuner of the batched sweeps (no counterpart in the reference). For each
  * direction it times the persistent first-stage sweep of the whole batch over
  * the tilings it can run: tile shape in cells per chunk x lines per CTA
- * (0: 16 x 8 along x, 32 x 4 in the 2D mixed form, 8 x 16 along y and z; 1:
- * 32 x 4 along x, 8 x 32 along y and z, 2D and 3D FP64 only), lines cut into
+ * (2D and 3D FP64: 0 is 32 x 4 along x and 8 x 32 along y and z, 1, which a
+ * batch starts with, 16 x 8 along x and 8 x 16 along y and z; the mixed form
+ * and 1D have one shape, 0), lines cut into
  * 1, 2, 4 or 8 segments, and one or as many persistent CTAs per SM as fit;
  * keeps the fastest. Results are bit for bit those of any other tiling. The tuning runs
  * sweeps on the cases' current states and touches only scratch buffers (RHS,
