@@ -2063,9 +2063,14 @@ int cfd_batch_autotune(cfd_batch *b, int *choice, double *ms)
     for (int d = 0; d < b->dim && rc == CFD_OK; d++) {
         float best = 3.4e38f;
         int best_cfg[3] = {b->shape[d], b->split[d], b->one_cta[d]};
+        // the powers of two the default is chosen from, and the segments the
+        // batch has now if those are others
+        std::vector<int> splits = {1, 2, 4, 8, 16};
+        if (std::find(splits.begin(), splits.end(), b->split[d]) == splits.end()) splits.push_back(b->split[d]);
         for (int shape = 0; shape <= (alt ? 1 : 0) && rc == CFD_OK; shape++)
-            for (int split = 1; split <= 8 && rc == CFD_OK; split *= 2)
+            for (size_t s = 0; s < splits.size() && rc == CFD_OK; s++)
                 for (int one = 0; one <= 1 && rc == CFD_OK; one++) {
+                    const int split = splits[s];
                     b->shape[d] = shape;
                     b->split[d] = split;
                     b->one_cta[d] = one;

@@ -296,8 +296,8 @@ int cfd_batch_run(cfd_batch *b, double cfl, int end_step, const double *output_d
  * (2D and 3D FP64: 0 is 32 x 4 along x and 8 x 32 along y and z, 1, which a
  * batch starts with, 16 x 8 along x and 8 x 16 along y and z; the mixed form
  * and 1D have one shape, 0), lines cut into
- * 1, 2, 4 or 8 segments, and one or as many persistent CTAs per SM as fit;
- * keeps the fastest. Results are bit for bit those of any other tiling. The tuning runs
+ * 1, 2, 4, 8 or 16 segments or as many as they are cut into already, and one
+ * or as many persistent CTAs per SM as fit; keeps the fastest. Results are bit for bit those of any other tiling. The tuning runs
  * sweeps on the cases' current states and touches only scratch buffers (RHS,
  * stage state); call it between runs. choice (may be NULL) receives per
  * direction {shape, segments, one CTA per SM}, ms (may be NULL) the chosen
