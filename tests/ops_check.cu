@@ -2,6 +2,7 @@
 // for tests/test_gpu_ops.py: operand rows in, result rows out, beside the
 // compiler's own operations where a comparison needs them.
 #include "adjoint_math.h"
+#include "euler_math.cuh"
 
 #include <cuda_runtime.h>
 
@@ -42,6 +43,18 @@ struct FaceVjp {  // six cells' cons and the adjoint of the flux, along x
     }
 };
 
+#if defined(CFD_FAST)
+struct Wcns5Pair {  // a field's six values: both face states, whether the fast path took them
+    static constexpr int in = 6, out = 3;
+    static __device__ void f(const double *x, double *r)
+    {
+        cfd::OpsSpec o;
+        cfd::wcns5_pair(x, r[0], r[1], o);
+        r[2] = o.ok;
+    }
+};
+#endif
+
 template <class OP>
 __global__ void each(const double *x, double *r, long n)
 {
@@ -71,5 +84,8 @@ extern "C" {
 int ops_arcp(const double *x, double *r, long n) { return run<Arcp>(x, r, n); }
 int ops_asqrt(const double *x, double *r, long n) { return run<Asqrt>(x, r, n); }
 int ops_wcns5_adj(const double *x, double *r, long n) { return run<Wcns5Adj>(x, r, n); }
+#if defined(CFD_FAST)
+int ops_wcns5_pair(const double *x, double *r, long n) { return run<Wcns5Pair>(x, r, n); }
+#endif
 int ops_face_vjp(const double *x, double *r, long n) { return run<FaceVjp>(x, r, n); }
 }

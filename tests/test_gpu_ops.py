@@ -132,3 +132,42 @@ def test_face_density_that_cancels(ops):
         for k in range(-40, 41):
             rows.append([*cells(lo + k * np.spacing(lo)).ravel(), *rng.normal(size=4)])
     assert np.isfinite(ops("fast", "face_vjp", rows, 24)).all()
+
+
+def wcns5(q):
+    """weno5_JSchen in extended precision, one row of five values a result."""
+    q = q.astype(np.longdouble).T
+    s = [(q[0] - 2 * q[1] + q[2])**2 + (q[0] - 4 * q[1] + 3 * q[2])**2 / 4,
+         (q[1] - 2 * q[2] + q[3])**2 + (q[1] - q[3])**2 / 4,
+         (q[2] - 2 * q[3] + q[4])**2 + (3 * q[2] - 4 * q[3] + q[4])**2 / 4]
+    w = [g / (np.longdouble(1e-6) + b)**2 for g, b in zip((1 / 16, 5 / 8, 5 / 16), s)]
+    u = [0.375 * q[0] - 1.25 * q[1] + 1.875 * q[2], -0.125 * q[1] + 0.75 * q[2] + 0.375 * q[3],
+         0.375 * q[2] + 0.75 * q[3] - 0.125 * q[4]]
+    return sum(a * b for a, b in zip(w, u)) / sum(w)
+
+
+@pytest.mark.parametrize("amplitude", [1e-6, 1e-2, 1.0, 1e4, 1e7, 1e9, 1e12, 1e25])
+def test_fast_wcns5_pair(ops, amplitude):
+    """Both states of a face from shared differences, for differences from the
+    smallest to shocks in SI units: taken by the branch-free path and within
+    rounding of extended precision. A weight's relative error is below 64
+    roundings (its measure's, squared, times another), which moves the mean of
+    candidates by as many roundings of twice their spread of ten differences."""
+    rng = np.random.default_rng(6)
+    q = rng.normal(size=(20000, 6)) * amplitude
+    jump = rng.integers(1, 6, len(q))
+    q += (np.arange(6) >= jump[:, None]) * amplitude * 10
+    q[::4] = np.where(np.arange(6) >= jump[::4, None], amplitude, 0.0)  # one clean jump
+    r = ops("fast", "wcns5_pair", q, 3)
+    assert (r[:, 2] == 1).all()
+    spread = np.abs(np.diff(q, axis=1)).max(1)
+    tol = 64 * 2 * 10 * 2.0**-53 * spread + 2.0**-52 * np.abs(q).max(1)
+    assert (np.abs(r[:, 0] - wcns5(q[:, :5])) <= tol).all()
+    assert (np.abs(r[:, 1] - wcns5(q[:, :0:-1])) <= tol).all()
+
+
+def test_fast_wcns5_pair_leaves_what_it_does_not_cover(ops):
+    """Differences whose measures leave the range, infinities and NaN."""
+    q = np.zeros((5, 6))
+    q[:, 3:] = np.array([1e40, 1e80, 1e160, INF, NAN])[:, None]
+    assert (ops("fast", "wcns5_pair", q, 3)[:, 2] == 0).all()
