@@ -175,36 +175,41 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
         const double got = cfd::div_rn(a, b, y), want = a / b;
         if (__double_as_longlong(got) != __double_as_longlong(want) || __double_as_longlong(y) != __double_as_longlong(1.0 / b))
             cnt++;
-        // the sweeps' branch-free operations where they accept the operands:
-        // the pair above, and operands next to the ends of a binade (all-ones
-        // significands, one ulp above a power of two) where a reciprocal or a
-        // root lies nearest a rounding boundary
+        // the sweeps' branch-free operations: they have to accept exactly the
+        // operands of their ranges, and to round as IEEE wherever they do. The
+        // pair above, divisors and dividends over the ranges and a few binades
+        // beyond, and significands next to the ends of a binade, where a
+        // reciprocal or a root lies nearest a rounding boundary; the first 608
+        // pairs take the all-ones significand through every exponent.
         {
-            const unsigned long long k = splitmix64(st) % 8;
-            const int e = (int)(splitmix64(st) % 121) - 60;
-            const unsigned long long m = (1ULL << 52) - 1, low = splitmix64(st) % 16;
-            const unsigned long long mant = (k == 0) ? m - low : (k == 1) ? low : (splitmix64(st) & m);
+            const unsigned long long k = splitmix64(st) % 8, m = (1ULL << 52) - 1, low = splitmix64(st) % 16;
+            const int e = i < 608 ? (int)i - 404 : (k & 1) ? (int)(splitmix64(st) % 121) - 60 : (int)(splitmix64(st) % 608) - 404;
+            const unsigned long long mant = i < 608 ? m : (k < 2) ? m - low : (k < 4) ? low : (splitmix64(st) & m);
             const double bs = __longlong_as_double((long long)(((unsigned long long)(1023 + e) << 52) | mant));
-            const double bp = (k < 4) ? bs : b;
-            {
+            const double bp = (i < 608 || k < 6) ? bs : b;
+            const double ae = (splitmix64(st) & 1) ? rand_double(st, -804, -797) : rand_double(st, 496, 503);
+            auto within = [](double x, int lo, int hi) { return x != 0.0 && ilogb(x) >= lo && ilogb(x) < hi; };
+            auto same = [](double x, double w) { return __double_as_longlong(x) == __double_as_longlong(w); };
+            const bool b_in = within(bp, -400, 200);
+            for (int j = 0; j < 2; j++) {
+                const double aj = j ? ae : a;
+                const bool a_in = aj == 0.0 || within(aj, -800, 500);
                 cfd::OpsSpec o;
                 const double r = o.rcp(bp);
-                if (o.ok && __double_as_longlong(r) != __double_as_longlong(1.0 / bp)) cnt++;
-                const double q = o.div_y(a, bp, r);
-                if (o.ok && __double_as_longlong(q) != __double_as_longlong(a / bp)) cnt++;
+                if (o.ok != b_in || (o.ok && !same(r, 1.0 / bp))) cnt++;
+                const double q = o.div_y(aj, bp, r);
+                if (o.ok != (b_in && a_in) || (o.ok && !same(q, aj / bp))) cnt++;
+                cfd::OpsSpec o2;
+                const double q2 = o2.div(aj, bp);
+                if (o2.ok != (b_in && a_in) || (o2.ok && !same(q2, aj / bp))) cnt++;
             }
-            {
-                cfd::OpsSpec o;
-                const double q = o.div(a, bp);
-                if (o.ok && __double_as_longlong(q) != __double_as_longlong(a / bp)) cnt++;
-            }
-            {  // roots: as above, and next to the square of a rounding boundary
-                const double s = fabs(bp), hu = ldexp(1.0, ilogb(s) - 53);
-                const double x = (k & 1) ? fma(s, s, s * (2.0 * hu)) : s;
-                cfd::OpsSpec o;
-                const double r = o.sqrt(x);
-                if (o.ok && __double_as_longlong(r) != __double_as_longlong(sqrt(x))) cnt++;
-            }
+            // roots: of bp, and next to the square of a rounding boundary
+            const double hu = ldexp(1.0, ilogb(bp) - 53), x = (k & 1) ? fma(bp, bp, bp * (2.0 * hu)) : bp;
+            cfd::OpsSpec o;
+            const double r = o.sqrt(x);
+            if (o.ok != within(x, -400, 200) || (o.ok && !same(r, sqrt(x)))) cnt++;
+            // the unchecked root takes products of two densities and pressure ratios
+            if (within(x, -800, 600) && !same(cfd::OpsSpec().sqrt_in(x), sqrt(x))) cnt++;
         }
     }
     if (cnt) atomicAdd(bad, cnt);

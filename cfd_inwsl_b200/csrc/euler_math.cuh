@@ -143,7 +143,8 @@ static __device__ __noinline__ DivN<N> divs_ieee(DivN<N> a, DivN<N> b)
 // 34(1), 1990). y comes from the hardware's reciprocal approximation by one
 // cubic (Halley) step, 1/b (1 - e^3) for a seed off by e; a further Markstein
 // step makes it RN(1/b) where 1/b itself is wanted. The root is Markstein's
-// s + (x - s^2) / (2 sqrt x) on a seed after one cubic step. Division: 6
+// s + (x - s^2) / (2 sqrt x) on a seed after one cubic step. The all-ones
+// significand rests on the seed itself (rcp_near). Division: 6
 // operations on the FP64 pipe instead of about 14 issue slots and a branch;
 // cfd_check_division compares all of them with IEEE on the device.
 // Fast flavour: the same steps without the last correction where its own
@@ -195,9 +196,13 @@ struct OpsSpec {
         return (t - (223u << 20) < (1300u << 20)) | ((t | lo) == 0u);
     }
     // 1/b to just over half an ulp: seed (relative error e) and y (1 + e + e^2).
-    // e + e^2 is rounded up: for a significand of all ones 1/b lies 2^-107
-    // above a rounding boundary, the one case in which the Markstein step
-    // does not recover from the neighbour below.
+    // The Markstein step that follows recovers RN(1/b) from either neighbour,
+    // except for a significand of all ones: there 1/b lies 2^-107 above a
+    // rounding boundary, and y must not end below it. e + e^2 rounded up keeps
+    // it above for |e| < 2^-26 only; a seed above 1/b (e < 0) does so for any
+    // e, since y (1 + e + e^2) = (1 - e^3) / b. That is a property of this
+    // chip's seed for that one significand, as is the root of an all-ones
+    // radicand, and cfd_check_division tests it for every exponent in range.
     static __device__ __forceinline__ double rcp_near(double b)
     {
         double y;

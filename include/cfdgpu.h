@@ -212,10 +212,12 @@ int cfd_fp64_peak_probe(long long iters, void *stream, double *flops);
  * reciprocal (Markstein's correction) against the device's IEEE division on n
  * seeded operand pairs (random, next to rounding midpoints, physical ranges,
  * signed zeros, tiny and huge dividends), and of the sweeps' branch-free
- * quotients, reciprocals and square roots where they accept the operands
- * (significands next to the ends of a binade and squares next to rounding
- * boundaries among them); *mismatches counts results whose bits differ. No counterpart in the reference: it
- * backs the strict flavour's bit-for-bit parity. */
+ * quotients, reciprocals and square roots over their ranges and a little
+ * beyond (significands next to the ends of a binade, the all-ones one at every
+ * exponent, and squares next to rounding boundaries among them). *mismatches
+ * counts results whose bits differ, operands in range that the branch-free
+ * operations refuse and others that they take. No counterpart in the
+ * reference: it backs the strict flavour's bit-for-bit parity. */
 int cfd_check_division(long long n, unsigned long long seed, unsigned long long *mismatches);
 
 /* Pointwise known-answer hooks: evaluate the device interpolator for

@@ -43,7 +43,34 @@ struct FaceVjp {  // six cells' cons and the adjoint of the flux, along x
     }
 };
 
+// operands a and b, b > 0: branch-free a/b, 1/b, sqrt(b), each followed by
+// whether it was taken and by the compiler's
+struct Spec {
+    static constexpr int in = 2, out = 9;
+    static __device__ void f(const double *x, double *r)
+    {
+        cfd::OpsSpec q, y, s;
+        r[0] = q.div(x[0], x[1]);
+        r[1] = q.ok;
+        r[2] = x[0] / x[1];
+        r[3] = y.rcp(x[1]);
+        r[4] = y.ok;
+        r[5] = 1.0 / x[1];
+        r[6] = s.sqrt(x[1]);
+        r[7] = s.ok;
+        r[8] = sqrt(x[1]);
+    }
+};
 #if defined(CFD_FAST)
+struct Rsqrt {
+    static constexpr int in = 1, out = 2;
+    static __device__ void f(const double *x, double *r)
+    {
+        cfd::OpsSpec o;
+        r[0] = o.rsqrt(x[0]);
+        r[1] = o.ok;
+    }
+};
 struct Wcns5Pair {  // a field's six values: both face states, whether the fast path took them
     static constexpr int in = 6, out = 3;
     static __device__ void f(const double *x, double *r)
@@ -81,10 +108,12 @@ int run(const double *x, double *r, long n)
 } // namespace
 
 extern "C" {
+int ops_spec(const double *x, double *r, long n) { return run<Spec>(x, r, n); }
 int ops_arcp(const double *x, double *r, long n) { return run<Arcp>(x, r, n); }
 int ops_asqrt(const double *x, double *r, long n) { return run<Asqrt>(x, r, n); }
 int ops_wcns5_adj(const double *x, double *r, long n) { return run<Wcns5Adj>(x, r, n); }
 #if defined(CFD_FAST)
+int ops_rsqrt(const double *x, double *r, long n) { return run<Rsqrt>(x, r, n); }
 int ops_wcns5_pair(const double *x, double *r, long n) { return run<Wcns5Pair>(x, r, n); }
 #endif
 int ops_face_vjp(const double *x, double *r, long n) { return run<FaceVjp>(x, r, n); }

@@ -54,6 +54,59 @@ def normals(rng, n, lo, hi):
     return np.ldexp(m, rng.integers(lo, hi, n))
 
 
+def spec_operands():
+    """Dividends and divisors in range with exponents from end to end, the
+    all-ones significand and its neighbours at every exponent, zeros."""
+    rng = np.random.default_rng(0)
+    n = 1 << 20
+    b = normals(rng, n, -400, 200)
+    a = normals(rng, n, -800, 500) * rng.choice([-1.0, 1.0], n)
+    e = np.arange(-400, 200)
+    edge = np.concatenate([np.ldexp(2 - k * 2.0**-52, e) for k in (1, 2, 3)] + [np.ldexp(1 + k * 2.0**-52, e) for k in (0, 1, 2)])
+    ends_a = np.ldexp(rng.uniform(1, 2, 64), np.resize([-800, -799, 498, 499], 64))
+    b = np.concatenate([b, edge, edge, np.repeat(edge, 64)])
+    a = np.concatenate([a, np.zeros(len(edge)), -np.zeros(len(edge)), np.tile(ends_a, len(edge))])
+    return np.stack([a, b], 1)
+
+
+def test_branch_free_operations_strict(ops):
+    """Taken for every operand in range and rounded as the compiler's."""
+    x = spec_operands()
+    r = ops("strict", "spec", x, 9)
+    assert (r[:, [1, 4, 7]] == 1).all()
+    for k in (0, 3, 6):
+        np.testing.assert_array_equal(r[:, k].view(np.uint64), r[:, k + 2].view(np.uint64))
+
+
+def test_branch_free_operations_fast(ops):
+    """The same operations in the fast flavour: quotients and roots keep their
+    correction; its reciprocal is the cubic step alone, within an ulp, and its
+    reciprocal root within 1.5 roundings of 2^-53 (the residual's product and
+    the result's) and the step's own error."""
+    x = spec_operands()
+    r = ops("fast", "spec", x, 9)
+    assert (r[:, [1, 4, 7]] == 1).all()
+    for k in (0, 3, 6):
+        assert (np.abs(r[:, k] - r[:, k + 2]) <= np.spacing(np.abs(r[:, k + 2]))).all()
+    b = x[:, 1]
+    r = ops("fast", "rsqrt", b[:, None], 2)
+    assert (r[:, 1] == 1).all()
+    want = 1 / np.sqrt(b.astype(np.longdouble))
+    assert (np.abs(r[:, 0] - want) <= (1.5 * 2.0**-53 + 2.0**-56) * want).all()
+
+
+@pytest.mark.parametrize("flavour", ["strict", "fast"])
+def test_branch_free_operations_leave_other_operands(ops, flavour):
+    """Operands outside the ranges, next to their ends among them, are refused:
+    the callers evaluate those out of line."""
+    below, above = np.nextafter(2.0**-400, 0), 2.0**200
+    for v in (below, 2.0**-401, above, 2.0**201, 0.0, -0.0, -1.0, INF, NAN, 5e-324):
+        r = ops(flavour, "spec", [[1.0, v]], 9)[0]
+        assert (r[[1, 4, 7]] == 0).all(), v
+    for v in (np.nextafter(2.0**-800, 0), 5e-324, -(2.0**-801), 2.0**500, -(2.0**501), INF, NAN):
+        assert ops(flavour, "spec", [[v, 1.0]], 9)[0, 1] == 0, v
+
+
 def test_adjoint_reciprocal_and_root(ops):
     """Within an ulp of the compiler's for normal operands: a cubic step from a
     seed off by less than 2^-18 leaves 2^-54, and one rounding half an ulp."""
