@@ -168,3 +168,18 @@ def test_trad6_five_ghosts(periodic):
         return zone.BlockSolver(info, periodic=periodic)
 
     compare(make, c, 0.5)
+
+
+@pytest.mark.parametrize("flavour", ["strict", "fast", "mixed"])
+@pytest.mark.parametrize("n,periodic", [((520, 869), True), ((700, 410), False), ((40, 36, 70), True)])
+def test_default_segments_of_chunks(n, periodic, flavour):
+    """Chunk launches cut their own segments where the configuration gives
+    none: 16 instead of 72 rows along the last direction of 520 x 869 (32
+    instead of 144 cells along x, in the strict flavour 13 by the one-chunk
+    kernel), 8 instead of 48 of 700 x 410, 8 instead of 24 planes of 40 x 36 x
+    70, a remainder left by each."""
+    dim = len(n)
+    c = (smooth_2d(*n, np.random.default_rng(31)) if dim == 2 else smooth_state_3d(n, np.random.default_rng(31)))
+    make = lambda: gpu_solver(dim, list(n), im=11 if dim == 2 else 2, fm=dim == 2, periodic=periodic, cfl=0.4,
+                              strict=flavour == "strict", precision=int(flavour == "mixed"))
+    compare(make, c, 0.4, steps=2)
