@@ -61,6 +61,27 @@ struct Spec {
         r[8] = sqrt(x[1]);
     }
 };
+struct DivSum {  // a / b for a sum of weights b >= 1, whether it was taken, the compiler's
+    static constexpr int in = 2, out = 3;
+    static __device__ void f(const double *x, double *r)
+    {
+        cfd::OpsSpec o;
+        r[0] = o.div_sum(x[0], x[1]);
+        r[1] = o.ok;
+        r[2] = x[0] / x[1];
+    }
+};
+struct Wenoz {  // five stencil values: WENO-Z, whether the branch-free path took them, by the compiler's operations
+    static constexpr int in = 5, out = 3;
+    static __device__ void f(const double *x, double *r)
+    {
+        cfd::OpsSpec o;
+        cfd::OpsIeee i;
+        r[0] = cfd::inter5<cfd::FAM_WENOZ>(x[0], x[1], x[2], x[3], x[4], 0.0, 0.0, o);
+        r[1] = o.ok;
+        r[2] = cfd::inter5<cfd::FAM_WENOZ>(x[0], x[1], x[2], x[3], x[4], 0.0, 0.0, i);
+    }
+};
 #if defined(CFD_FAST)
 struct Rsqrt {
     static constexpr int in = 1, out = 2;
@@ -108,6 +129,8 @@ int run(const double *x, double *r, long n)
 } // namespace
 
 extern "C" {
+int ops_div_sum(const double *x, double *r, long n) { return run<DivSum>(x, r, n); }
+int ops_wenoz(const double *x, double *r, long n) { return run<Wenoz>(x, r, n); }
 int ops_spec(const double *x, double *r, long n) { return run<Spec>(x, r, n); }
 int ops_arcp(const double *x, double *r, long n) { return run<Arcp>(x, r, n); }
 int ops_asqrt(const double *x, double *r, long n) { return run<Asqrt>(x, r, n); }

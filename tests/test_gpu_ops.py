@@ -107,6 +107,47 @@ def test_branch_free_operations_leave_other_operands(ops, flavour):
         assert ops(flavour, "spec", [[v, 1.0]], 9)[0, 1] == 0, v
 
 
+def test_division_by_a_sum_of_weights(ops):
+    """WENO-Z's last division: taken and rounded as the compiler's while the
+    quotient is 0 or within 2^-960 .. 2^1000, refused next to and beyond the
+    ends (a refused one is only computed again)."""
+    rng = np.random.default_rng(7)
+    b = normals(rng, 1 << 20, 0, 1000)
+    q = normals(rng, 1 << 20, -959, 20) * rng.choice([-1.0, 1.0], 1 << 20)
+    q[:1000], q[1000:2000] = 0.0, -0.0
+    edge = np.concatenate([np.ldexp(2 - k * 2.0**-52, np.arange(1000)) for k in (1, 2)] + [np.ldexp(1.0, np.arange(1000))])
+    b = np.concatenate([b, edge])
+    a = np.concatenate([q, rng.normal(size=len(edge))]) * b
+    r = ops("strict", "div_sum", np.stack([a, b], 1), 3)
+    assert (r[:, 1] == 1).all()
+    np.testing.assert_array_equal(r[:, 0].view(np.uint64), r[:, 2].view(np.uint64))
+    bad = [[1.0, 2.0**1000], [1.0, INF], [1.0, NAN], [NAN, 1.0], [INF, 1.0], [1e-300, 2.0**600], [2.0**1010, 1.0]]
+    assert (ops("strict", "div_sum", bad, 3)[:, 1] == 0).all()
+
+
+@pytest.mark.parametrize("flavour", ["strict", "fast"])
+def test_wenoz_beside_a_flat_side(ops, flavour):
+    """Stencils of equal values, with a jump or noise beside them: a weight
+    there is the square of the jump's measure over 1e-40 and was refused, so
+    that the whole face was computed twice. Taken, and equal to the compiler's
+    operations (strict) or within the spread's rounding (fast: its quotients
+    are the same, sums are contracted)."""
+    rng = np.random.default_rng(8)
+    q = np.ones((20000, 5)) * rng.normal(size=(20000, 1))
+    jump = rng.integers(1, 5, len(q))
+    size = rng.normal(size=(len(q), 1)) * 10.0**rng.integers(-12, 9, (len(q), 1))
+    q += (np.arange(5) >= jump[:, None]) * size
+    q[::3] += 1e-15 * rng.normal(size=(len(q[::3]), 5))
+    r = ops(flavour, "wenoz", q, 3)
+    assert (r[:, 1] == 1).all()
+    if flavour == "strict":
+        np.testing.assert_array_equal(r[:, 0].view(np.uint64), r[:, 2].view(np.uint64))
+    else:
+        # two evaluations of one formula: candidates within 8 roundings of the
+        # stencil's largest value each, weights positive
+        assert (np.abs(r[:, 0] - r[:, 2]) <= 16 * 2.0**-52 * np.abs(q).max(1)).all()
+
+
 def test_adjoint_reciprocal_and_root(ops):
     """Within an ulp of the compiler's for normal operands: a cubic step from a
     seed off by less than 2^-18 leaves 2^-54, and one rounding half an ulp."""
